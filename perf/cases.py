@@ -439,7 +439,9 @@ def tolerance(case):
         return {"rel": 1e-5} if case["mode"] == 0 else {"rel": 4e-3}
     if kind == "mlp_predict":
         return {"rel": 4e-3}
-    return {"rel": 1e-2}
+    # Adam divides small gradients by their own size: the same path with its sums in another order
+    # moved the weights by 8e-4 of their norm, single ones by 0.03 of their root mean square
+    return {"rel": 3.5e-3, "max": 0.13}
 
 
 # ------------------------------------------------------------------------------ in 64 bits
