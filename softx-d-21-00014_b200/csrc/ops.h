@@ -114,10 +114,18 @@ void cheby_step(const DCsr &A, const F *t1s, const F *rs, const F *isd, F c, F *
 void prolong_mixed(const DCsr &P, const float *xH, double *x, bool x_zero, int nv,
                    cudaStream_t s);
 
-// HSGS: forward+backward sweeps over GS blocks (t = b - A_off x_old given)
+// HSGS: forward+backward sweeps over the Gauss-Seidel blocks. t is b -
+// A_offblock x_old; xin is x itself, or null for a sweep from x = 0 (t is then
+// b). plan: the blocks' sizes.
+struct HsgsPlan {
+    uint64_t n = 0;
+    uint32_t rows = 0;        // rows of a block (the last one may be shorter)
+    uint32_t ent_max[6] = {}; // most in-block entries of 2^l consecutive blocks
+};
 template <typename F>
-void hsgs_sweep(const DCsr &Adiag, const uint64_t *boff, int nblocks, const F *t, F *x,
-                const F *d, const double *relax_sc, int nv, cudaStream_t s);
+void hsgs_sweep(const DCsr &Adiag, const HsgsPlan &plan, const uint64_t *boff, int nblocks,
+                const F *t, const F *xin, F *x, const F *d, const double *relax_sc, int nv,
+                cudaStream_t s);
 
 // Dense y = A_inv x (Direct coarse solve)
 template <typename F>

@@ -1,0 +1,86 @@
+// Launchers of the block smoother (hybrid symmetric Gauss-Seidel) and the dense
+// coarse solve.
+#include "hsgs.cuh"
+#include "spmv_launch.cuh"
+
+namespace xg {
+namespace ops {
+
+// Gauss-Seidel blocks a thread block takes (group): one warp of lanes at
+// most (group * nv <= 32); fewer while the grid would not fill the GPU twice,
+// since a block of rows is one serial chain and a lane waits for its warp's
+// longest row. A block of rows that does not fit in shared memory
+// (gpu_hsgs_rows of many hundreds) is swept from global memory.
+constexpr uint32_t HS_SMEM_MAX = 96u * 1024u;
+
+template <typename F, typename I, int NV>
+static bool hsgs_shape(const HsgsPlan &p, k::HsgsShape &sh) {
+    int l = NV >= 32 ? 0 : NV >= 16 ? 1 : NV >= 8 ? 2 : NV >= 4 ? 3 : NV >= 2 ? 4 : 5;
+    for (; l >= 0; --l) {
+        sh = k::HsgsShape{p.n, p.rows, 1u << l, p.ent_max[l]};
+        const uint64_t grid = (p.n + (uint64_t)p.rows * sh.group - 1) / ((uint64_t)p.rows * sh.group);
+        const uint64_t values = (uint64_t)(p.rows + 1) * sh.group * NV + p.ent_max[l];
+        if (values < HS_SMEM_MAX && k::hs_smem_bytes<F, I, NV>(sh) <= HS_SMEM_MAX &&
+            (l == 0 || grid >= 2ull * (uint64_t)ctx().sms))
+            return true;
+    }
+    return false;
+}
+
+template <typename F>
+void hsgs_sweep(const DCsr &A, const HsgsPlan &plan, const uint64_t *boff, int nblocks,
+                const F *t, const F *xin, F *x, const F *d, const double *relax_sc, int nv,
+                cudaStream_t s) {
+    if (nblocks == 0 || A.nrows == 0) return;
+    XG_DISPATCH(A, nv, {
+        k::HsgsShape sh;
+        if (hsgs_shape<F, I, NV>(plan, sh)) {
+            auto kern = k::k_hsgs_block<F, I, NV>;
+            const uint32_t smem = k::hs_smem_bytes<F, I, NV>(sh);
+            static bool big_smem = false;  // one flag per instantiation
+            if (!big_smem) {
+                XG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)HS_SMEM_MAX));
+                big_smem = true;
+            }
+            const uint64_t per = (uint64_t)sh.rows * sh.group;
+            kern<<<(unsigned)((A.nrows + per - 1) / per), k::HS_THREADS, smem, s>>>(
+                A.row.as<uint32_t>(), (const I *)A.col.p, A.val.as<F>(), sh, t, xin, x, d,
+                relax_sc);
+        } else {
+            if (!xin) fill<F>(x, A.nrows * (uint64_t)NV, F(0), s);
+            const uint64_t threads = (uint64_t)nblocks * NV;
+            const int B = (int)((threads + k::CT - 1) / k::CT);
+            k::k_hsgs_sweep<F, I, NV><<<B, k::CT, 0, s>>>(A.row.as<uint32_t>(),
+                                                          (const I *)A.col.p, A.val.as<F>(), boff,
+                                                          nblocks, t, x, d, relax_sc);
+        }
+        XG_CUDA(cudaGetLastError());
+        ++g_kernel_launches;
+    });
+}
+template void hsgs_sweep<double>(const DCsr &, const HsgsPlan &, const uint64_t *, int,
+                                 const double *, const double *, double *, const double *,
+                                 const double *, int, cudaStream_t);
+template void hsgs_sweep<float>(const DCsr &, const HsgsPlan &, const uint64_t *, int,
+                                const float *, const float *, float *, const float *,
+                                const double *, int, cudaStream_t);
+
+template <typename F>
+void dense_apply(const F *a, uint64_t n, const F *x, F *y, int nv, cudaStream_t s) {
+    if (n == 0) return;
+    dispatch_nv(nv, [&](auto nvc) {
+        constexpr int NV = decltype(nvc)::value;
+        constexpr uint64_t RB = k::DT / NV;
+        k::k_dense<F, NV><<<(unsigned)((n + RB - 1) / RB), k::DT, 0, s>>>(a, n, x, y);
+        XG_CUDA(cudaGetLastError());
+        ++g_kernel_launches;
+    });
+}
+template void dense_apply<double>(const double *, uint64_t, const double *, double *, int,
+                                  cudaStream_t);
+template void dense_apply<float>(const float *, uint64_t, const float *, float *, int,
+                                 cudaStream_t);
+
+}  // namespace ops
+}  // namespace xg

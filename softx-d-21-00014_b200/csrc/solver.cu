@@ -195,6 +195,7 @@ struct Hsgs : public SolverBase {
     DevBuf d, boff, relax_dev;
     std::vector<double> relax_on_dev;  // what relax_dev holds (host mirror)
     DCsr Adiag, Aoff;
+    ops::HsgsPlan plan;
     int nblocks = 1;
     void setup_from(const HCsr &hA) {
         const uint64_t rows = cfg.gpu_hsgs_rows > 0 ? (uint64_t)cfg.gpu_hsgs_rows : 32;
@@ -239,6 +240,16 @@ struct Hsgs : public SolverBase {
             dg.row[i + 1] = (uint32_t)dg.col.size();
             od.row[i + 1] = (uint32_t)od.col.size();
         }
+        // blocks are cs rows each, the last one short (split_range_f64)
+        plan.n = n;
+        plan.rows = (uint32_t)std::min<uint64_t>(cs, n);
+        for (int l = 0; l < 6; ++l) {
+            const uint64_t per = (uint64_t)plan.rows << l;
+            plan.ent_max[l] = 0;
+            for (uint64_t r = 0; r < n; r += per)
+                plan.ent_max[l] = std::max(plan.ent_max[l],
+                                           dg.row[std::min(n, r + per)] - dg.row[r]);
+        }
         upload_csr(dg, Adiag, f32, cfg.gpu_index_compress, S());
         upload_csr(od, Aoff, f32, cfg.gpu_index_compress, S(), cfg.gpu_spmv_tune);
         upload(boff, off, S());
@@ -278,15 +289,13 @@ struct Hsgs : public SolverBase {
                 XG_CUDA(cudaMemcpyAsync(relax_dev.p, relax_on_dev.data(), NV * sizeof(double),
                                         cudaMemcpyHostToDevice, S()));
             }
-            if (x.zero) {
-                // no lagged term: t = 1*b + (-1)*0 = b; x = 0 (blas2.h:226-262)
-                ops::convert<F, F>(t.p<F>(), b.p<F>(), t.elems(), S());
-                ops::fill<F>(x.p<F>(), x.elems(), F(0), S());
-            } else {
+            // x zero-flagged: no lagged term, t = 1*b + (-1)*0 = b, and the
+            // sweep starts from x = 0 (blas2.h:226-262)
+            if (!x.zero)
                 ops::residual<F>(Aoff, x.p<F>(), b.p<F>(), t.p<F>(), NV, nullptr, S());
-            }
-            ops::hsgs_sweep<F>(Adiag, boff.as<uint64_t>(), nblocks, t.p<F>(), x.p<F>(), d.as<F>(),
-                               relax_dev.as<double>(), NV, S());
+            ops::hsgs_sweep<F>(Adiag, plan, boff.as<uint64_t>(), nblocks,
+                               x.zero ? b.p<F>() : t.p<F>(), x.zero ? nullptr : x.p<F>(),
+                               x.p<F>(), d.as<F>(), relax_dev.as<double>(), NV, S());
             x.zero = false;
             x.init = true;
             if (cfg.convergence_check) {
