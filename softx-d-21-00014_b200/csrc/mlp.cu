@@ -2,10 +2,12 @@
 // (n_in -> h -> h -> n_out, ReLU after the first two), BF16 weights and
 // activations with FP32 accumulation on the tcgen05 GEMM (gemm.cu), FP32
 // master weights trained with Adam on a mean-squared-error loss. Forward and
-// backward passes are GEMMs with fused epilogues plus a few element-wise
-// kernels here (transpose, loss gradient, bias gradient, Adam).
+// backward passes are GEMMs with fused epilogues (the loss gradient in the last
+// layer's), which read transposed operands where they lie, plus the bias
+// gradients and Adam here.
 #include <cuda_bf16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <random>
 
@@ -24,61 +26,88 @@ __global__ void k_f32_to_bf16(const float *__restrict__ in, __nv_bfloat16 *__res
         out[i] = __float2bfloat16_rn(in[i]);
 }
 
-// out[c][r] = in[r][c] for a rows x cols BF16 matrix (32 x 32 tiles)
-__global__ void k_transpose_bf16(const __nv_bfloat16 *__restrict__ in,
-                                 __nv_bfloat16 *__restrict__ out, uint32_t rows, uint32_t cols) {
-    __shared__ __nv_bfloat16 t[32][33];
-    const uint32_t c0 = blockIdx.x * 32, r0 = blockIdx.y * 32;
-    for (uint32_t j = threadIdx.y; j < 32; j += blockDim.y) {
-        const uint32_t r = r0 + j, c = c0 + threadIdx.x;
-        if (r < rows && c < cols) t[j][threadIdx.x] = in[(uint64_t)r * cols + c];
-    }
-    __syncthreads();
-    for (uint32_t j = threadIdx.y; j < 32; j += blockDim.y) {
-        const uint32_t c = c0 + j, r = r0 + threadIdx.x;
-        if (r < rows && c < cols) out[(uint64_t)c * rows + r] = t[threadIdx.x][j];
-    }
-}
-
-// dY = scale * (Y - T) in BF16; sum of squared errors into *sse
-__global__ void k_mse_grad(const float *__restrict__ Y, const float *__restrict__ T,
-                           __nv_bfloat16 *__restrict__ dY, uint64_t n, float scale, double *sse) {
-    double acc = 0.0;
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const float d = Y[i] - T[i];
-        acc += (double)d * d;
-        dY[i] = __float2bfloat16_rn(scale * d);
-    }
-    for (int off = 16; off; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
-    if ((threadIdx.x & 31) == 0) atomicAdd(sse, acc);
-}
-
-// db[c] = sum over rows of G[r][c] (BF16 in, FP32 out); one thread per column
-__global__ void k_colsum_bf16(const __nv_bfloat16 *__restrict__ G, float *__restrict__ db,
-                              uint32_t rows, uint32_t cols) {
-    const uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= cols) return;
+// Bias gradients of the three layers in one launch: db[c] = sum over rows of
+// G[r][c] in row order (BF16 in, FP32 out). A block copies 64 columns of up to
+// CS_ROWS rows at a time into shared memory (128 contiguous bytes a row, all
+// loads in flight) and 64 threads add their column from there. One thread
+// walking a whole column in global memory took 14 us a layer at 512 rows.
+struct ColSum {
+    const __nv_bfloat16 *g;
+    float *db;
+    uint32_t cols, block0;  // first block of this layer
+};
+struct ColSums {
+    ColSum l[3];
+};
+constexpr int CS_ROWS = 256, CS_THREADS = 256;
+__global__ void __launch_bounds__(CS_THREADS) k_colsum_bf16(ColSums a, uint32_t rows) {
+    __shared__ __align__(16) __nv_bfloat16 t[CS_ROWS][64];
+    const ColSum L = blockIdx.x >= a.l[2].block0   ? a.l[2]
+                     : blockIdx.x >= a.l[1].block0 ? a.l[1]
+                                                   : a.l[0];
+    const uint32_t c0 = (blockIdx.x - L.block0) * 64;
     float s = 0.f;
-    for (uint32_t r = 0; r < rows; ++r) s += __bfloat162float(G[(uint64_t)r * cols + c]);
-    db[c] = s;
+    for (uint32_t r0 = 0; r0 < rows; r0 += CS_ROWS) {
+        const uint32_t nr = rows - r0 < CS_ROWS ? rows - r0 : CS_ROWS;
+        if (r0) __syncthreads();
+#pragma unroll
+        for (int u = 0; u < CS_ROWS * 8 / CS_THREADS; ++u) {  // 16 bytes each
+            const uint32_t q = u * CS_THREADS + threadIdx.x, r = q / 8, p = q % 8;
+            if (r < nr)
+                reinterpret_cast<uint4 *>(t[r])[p] = __ldg(
+                    reinterpret_cast<const uint4 *>(L.g + (uint64_t)(r0 + r) * L.cols + c0) + p);
+        }
+        __syncthreads();
+        if (threadIdx.x < 64) {
+#pragma unroll 16
+            for (uint32_t r = 0; r < nr; ++r) s += __bfloat162float(t[r][threadIdx.x]);
+        }
+    }
+    if (threadIdx.x < 64) L.db[c0 + threadIdx.x] = s;
 }
 
-// Adam (Kingma & Ba 2015) on FP32 master parameters; bf16 receives the
-// rounded weights when given.
-__global__ void k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                       float *__restrict__ v, __nv_bfloat16 *__restrict__ bf16, uint64_t n,
-                       float lr, float b1, float b2, float eps, float c1, float c2) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.f - b1) * gi;
-        const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        const float pi = p[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-        p[i] = pi;
-        if (bf16) bf16[i] = __float2bfloat16_rn(pi);
+// Adam (Kingma & Ba 2015) on FP32 master parameters, every layer's weights and
+// biases in one launch, four values a thread; bf16 receives the rounded
+// weights. Bound by the 30 bytes a weight moves.
+struct AdamSeg {
+    float *p;
+    const float *g;
+    float *m, *v;
+    __nv_bfloat16 *bf16;  // null: none
+    uint64_t n4;          // values / 4
+};
+struct AdamSegs {
+    AdamSeg s[6];
+};
+__global__ void __launch_bounds__(256)
+    k_adam(AdamSegs a, float lr, float b1, float b2, float eps, float c1, float c2) {
+#pragma unroll 1
+    for (int q = 0; q < 6; ++q) {
+        const AdamSeg s = a.s[q];
+        for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < s.n4;
+             i += (uint64_t)gridDim.x * blockDim.x) {
+            float4 p4 = ((float4 *)s.p)[i], m4 = ((float4 *)s.m)[i], v4 = ((float4 *)s.v)[i];
+            const float4 g4 = ((const float4 *)s.g)[i];
+            float *p = &p4.x, *m = &m4.x, *v = &v4.x;
+            const float *g = &g4.x;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float gi = g[j];
+                const float mi = b1 * m[j] + (1.f - b1) * gi;
+                const float vi = b2 * v[j] + (1.f - b2) * gi * gi;
+                m[j] = mi;
+                v[j] = vi;
+                p[j] = p[j] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+            }
+            ((float4 *)s.p)[i] = p4;
+            ((float4 *)s.m)[i] = m4;
+            ((float4 *)s.v)[i] = v4;
+            if (s.bf16) {
+                alignas(8) const __nv_bfloat162 h[2] = {
+                    __floats2bfloat162_rn(p4.x, p4.y), __floats2bfloat162_rn(p4.z, p4.w)};
+                ((uint2 *)s.bf16)[i] = *reinterpret_cast<const uint2 *>(h);
+            }
+        }
     }
 }
 
@@ -116,31 +145,21 @@ void Mlp::init(uint32_t n_in_, uint32_t n_hidden, uint32_t n_out_, uint64_t seed
         for (DevBuf *z : {&L.mw, &L.vw, &L.mb, &L.vb})
             XG_CUDA(cudaMemsetAsync(z->p, 0, z->bytes, S()));
         L.wt_bf.alloc(nw * 2);
-        L.w_bf.alloc(nw * 2);
     }
     refresh_bf16();
     step = 0;
 }
 
-// BF16 copies of the weights: W^T as [out][in] for the forward pass, W as
-// [in][out] for the input gradients.
+// BF16 copy of the weights, W^T as [out][in]: the forward pass reads it as it
+// lies, the input gradients transposed.
 void Mlp::refresh_bf16() {
     for (Layer &L : layer) {
         const uint64_t nw = (uint64_t)L.out * L.in;
         k_f32_to_bf16<<<grid_for(nw), 256, 0, S()>>>(L.w.as<float>(),
                                                      L.wt_bf.as<__nv_bfloat16>(), nw);
-        transpose(L.wt_bf.p, L.w_bf.p, L.out, L.in);
         g_kernel_launches += 1;
     }
     XG_CUDA(cudaGetLastError());
-}
-
-void Mlp::transpose(const void *in, void *out, uint32_t rows, uint32_t cols) {
-    dim3 grid((cols + 31) / 32, (rows + 31) / 32), block(32, 8);
-    k_transpose_bf16<<<grid, block, 0, S()>>>((const __nv_bfloat16 *)in, (__nv_bfloat16 *)out,
-                                             rows, cols);
-    XG_CUDA(cudaGetLastError());
-    ++g_kernel_launches;
 }
 
 void Mlp::ensure(uint32_t batch) {
@@ -150,90 +169,115 @@ void Mlp::ensure(uint32_t batch) {
     cap = batch;
     const uint64_t B = batch;
     X.alloc(B * n_in * 2);
-    Xt.alloc(B * n_in * 2);
     H1.alloc(B * h * 2);
     H2.alloc(B * h * 2);
-    H1t.alloc(B * h * 2);
-    H2t.alloc(B * h * 2);
-    Y.alloc(B * n_out * 4);
     dY.alloc(B * n_out * 2);
-    dYt.alloc(B * n_out * 2);
     dH2.alloc(B * h * 2);
     dH1.alloc(B * h * 2);
-    dH2t.alloc(B * h * 2);
-    dH1t.alloc(B * h * 2);
-    sse.alloc(8);
+    const size_t parts = ops::mm::gemm_mse_parts(B, n_out);
+    sse.alloc(parts * sizeof(double));
+    if (sse_host) XG_CUDA(cudaFreeHost(sse_host));
+    sse_host = nullptr;
+    XG_CUDA(cudaMallocHost((void **)&sse_host, parts * sizeof(double)));
+    if (!sse_ready) XG_CUDA(cudaEventCreateWithFlags(&sse_ready, cudaEventDisableTiming));
 }
 
-void Mlp::forward(uint32_t batch, const float *Xf, float *Yout) {
+Mlp::~Mlp() {
+    if (sse_host) cudaFreeHost(sse_host);
+    if (sse_ready) cudaEventDestroy(sse_ready);
+}
+
+// The first two layers, activations kept in BF16.
+void Mlp::hidden(uint32_t batch, const float *Xf, bool split) {
     ensure(batch);
     const uint64_t B = batch;
     k_f32_to_bf16<<<grid_for(B * n_in), 256, 0, S()>>>(Xf, X.as<__nv_bfloat16>(), B * n_in);
     ++g_kernel_launches;
     using ops::mm::gemm_bf16;
     gemm_bf16(B, h, n_in, X.p, layer[0].wt_bf.p, H1.p, h, 2, layer[0].b.as<float>(), nullptr, 0,
-              S());
+              S(), false, false, split);
     gemm_bf16(B, h, h, H1.p, layer[1].wt_bf.p, H2.p, h, 2, layer[1].b.as<float>(), nullptr, 0,
-              S());
-    gemm_bf16(B, n_out, h, H2.p, layer[2].wt_bf.p, Yout ? (void *)Yout : Y.p, n_out, 0,
-              layer[2].b.as<float>(), nullptr, 0, S());
+              S(), false, false, split);
+}
+
+void Mlp::forward(uint32_t batch, const float *Xf, float *Yout) {
+    hidden(batch, Xf, true);
+    ops::mm::gemm_bf16(batch, n_out, h, H2.p, layer[2].wt_bf.p, Yout, n_out, 0,
+                       layer[2].b.as<float>(), nullptr, 0, S());
+}
+
+// Forward and backward pass; the partial sums of the loss are on their way to
+// the host when it returns (loss()). Its products never split their sums over
+// K: a step's weights depend on every rounding before it (Adam divides small
+// gradients by their own size), so training keeps one summation order whatever
+// the shapes.
+void Mlp::backward(uint32_t batch, const float *Xf, const float *T) {
+    hidden(batch, Xf, false);
+    const uint64_t B = batch;
+    using ops::mm::gemm_bf16;
+    const float scale = 2.0f / (float)(B * n_out);
+    // layer 3: dY and the loss from the forward product's epilogue; dW3^T = dY^T H2,
+    // dH2 = dY W3 masked by H2 > 0
+    sse_n = ops::mm::gemm_mse_grad(B, n_out, h, H2.p, layer[2].wt_bf.p, dY.p,
+                                   layer[2].b.as<float>(), T, scale, sse.as<double>(), S());
+    XG_CUDA(cudaMemcpyAsync(sse_host, sse.p, sse_n * sizeof(double), cudaMemcpyDeviceToHost, S()));
+    XG_CUDA(cudaEventRecord(sse_ready, S()));
+    gemm_bf16(n_out, h, B, dY.p, H2.p, layer[2].gw.p, h, 0, nullptr, nullptr, 0, S(), true, true,
+              false);
+    gemm_bf16(B, h, n_out, dY.p, layer[2].wt_bf.p, dH2.p, h, 3, nullptr, H2.p, h, S(), false, true,
+              false);
+    // layer 2
+    gemm_bf16(h, h, B, dH2.p, H1.p, layer[1].gw.p, h, 0, nullptr, nullptr, 0, S(), true, true,
+              false);
+    gemm_bf16(B, h, h, dH2.p, layer[1].wt_bf.p, dH1.p, h, 3, nullptr, H1.p, h, S(), false, true,
+              false);
+    // layer 1
+    gemm_bf16(h, n_in, B, dH1.p, X.p, layer[0].gw.p, n_in, 0, nullptr, nullptr, 0, S(), true, true,
+              false);
+    // bias gradients
+    ColSums cs;
+    cs.l[0] = ColSum{dY.as<__nv_bfloat16>(), layer[2].gb.as<float>(), n_out, 0};
+    cs.l[1] = ColSum{dH2.as<__nv_bfloat16>(), layer[1].gb.as<float>(), h, n_out / 64};
+    cs.l[2] = ColSum{dH1.as<__nv_bfloat16>(), layer[0].gb.as<float>(), h, (n_out + h) / 64};
+    k_colsum_bf16<<<(n_out + 2 * h) / 64, CS_THREADS, 0, S()>>>(cs, batch);
+    ++g_kernel_launches;
+    XG_CUDA(cudaGetLastError());
+}
+
+// The loss of the last backward pass (waits for its partial sums only).
+double Mlp::loss(uint32_t batch) {
+    XG_CUDA(cudaEventSynchronize(sse_ready));
+    double s = 0;
+    for (uint64_t i = 0; i < sse_n; ++i) s += sse_host[i];
+    return s / (double)((uint64_t)batch * n_out);
 }
 
 double Mlp::gradients(uint32_t batch, const float *Xf, const float *T) {
-    forward(batch, Xf, nullptr);
-    const uint64_t B = batch;
-    using ops::mm::gemm_bf16;
-    XG_CUDA(cudaMemsetAsync(sse.p, 0, 8, S()));
-    const float scale = 2.0f / (float)(B * n_out);
-    k_mse_grad<<<grid_for(B * n_out), 256, 0, S()>>>(Y.as<float>(), T, dY.as<__nv_bfloat16>(),
-                                                     B * n_out, scale, sse.as<double>());
-    ++g_kernel_launches;
-    // layer 3: dW3^T = dY^T H2, db3 = colsum dY, dH2 = (dY W3^T^T) masked by H2 > 0
-    transpose(dY.p, dYt.p, batch, n_out);
-    transpose(H2.p, H2t.p, batch, h);
-    gemm_bf16(n_out, h, B, dYt.p, H2t.p, layer[2].gw.p, h, 0, nullptr, nullptr, 0, S());
-    k_colsum_bf16<<<(n_out + 127) / 128, 128, 0, S()>>>(dY.as<__nv_bfloat16>(),
-                                                        layer[2].gb.as<float>(), batch, n_out);
-    gemm_bf16(B, h, n_out, dY.p, layer[2].w_bf.p, dH2.p, h, 3, nullptr, H2.p, h, S());
-    // layer 2
-    transpose(dH2.p, dH2t.p, batch, h);
-    transpose(H1.p, H1t.p, batch, h);
-    gemm_bf16(h, h, B, dH2t.p, H1t.p, layer[1].gw.p, h, 0, nullptr, nullptr, 0, S());
-    k_colsum_bf16<<<(h + 127) / 128, 128, 0, S()>>>(dH2.as<__nv_bfloat16>(),
-                                                    layer[1].gb.as<float>(), batch, h);
-    gemm_bf16(B, h, h, dH2.p, layer[1].w_bf.p, dH1.p, h, 3, nullptr, H1.p, h, S());
-    // layer 1
-    transpose(dH1.p, dH1t.p, batch, h);
-    transpose(X.p, Xt.p, batch, n_in);
-    gemm_bf16(h, n_in, B, dH1t.p, Xt.p, layer[0].gw.p, n_in, 0, nullptr, nullptr, 0, S());
-    k_colsum_bf16<<<(h + 127) / 128, 128, 0, S()>>>(dH1.as<__nv_bfloat16>(),
-                                                    layer[0].gb.as<float>(), batch, h);
-    g_kernel_launches += 3;
-    XG_CUDA(cudaGetLastError());
-    double s = 0;
-    XG_CUDA(cudaMemcpyAsync(&s, sse.p, 8, cudaMemcpyDeviceToHost, S()));
+    backward(batch, Xf, T);
     XG_CUDA(cudaStreamSynchronize(S()));
-    return s / (double)(B * n_out);
+    return loss(batch);
 }
 
 double Mlp::train_step(uint32_t batch, const float *Xf, const float *T, float lr) {
-    const double loss = gradients(batch, Xf, T);
+    backward(batch, Xf, T);
     ++step;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.f - std::pow(b1, (float)step), c2 = 1.f - std::pow(b2, (float)step);
-    for (Layer &L : layer) {
+    AdamSegs a;
+    uint64_t most = 0;
+    for (int l = 0; l < 3; ++l) {
+        Layer &L = layer[l];
         const uint64_t nw = (uint64_t)L.out * L.in;
-        k_adam<<<grid_for(nw), 256, 0, S()>>>(L.w.as<float>(), L.gw.as<float>(),
-                                              L.mw.as<float>(), L.vw.as<float>(), nullptr, nw, lr,
-                                              b1, b2, eps, c1, c2);
-        k_adam<<<grid_for(L.out), 256, 0, S()>>>(L.b.as<float>(), L.gb.as<float>(),
-                                                 L.mb.as<float>(), L.vb.as<float>(), nullptr,
-                                                 L.out, lr, b1, b2, eps, c1, c2);
-        g_kernel_launches += 2;
+        a.s[2 * l] = AdamSeg{L.w.as<float>(),  L.gw.as<float>(), L.mw.as<float>(),
+                             L.vw.as<float>(), L.wt_bf.as<__nv_bfloat16>(), nw / 4};
+        a.s[2 * l + 1] = AdamSeg{L.b.as<float>(),  L.gb.as<float>(), L.mb.as<float>(),
+                                 L.vb.as<float>(), nullptr, L.out / 4};
+        most = std::max(most, nw / 4);
     }
+    k_adam<<<grid_for(most), 256, 0, S()>>>(a, lr, b1, b2, eps, c1, c2);
+    ++g_kernel_launches;
     XG_CUDA(cudaGetLastError());
-    refresh_bf16();
-    return loss;
+    return loss(batch);
 }
 
 // Parameters in the order W1^T [h][in], b1, W2^T [h][h], b2, W3^T [out][h], b3.

@@ -12,17 +12,25 @@ struct Mlp {
         DevBuf w, b;          // FP32 master W^T [out][in], bias [out]
         DevBuf gw, gb;        // gradients (FP32)
         DevBuf mw, vw, mb, vb;  // Adam moments
-        DevBuf wt_bf, w_bf;   // BF16 W^T [out][in] and W [in][out]
+        DevBuf wt_bf;         // BF16 W^T [out][in]
     };
     uint32_t n_in = 0, h = 0, n_out = 0;
     Layer layer[3];
     uint64_t step = 0;
     uint32_t cap = 0;  // batch the activation buffers are sized for
-    DevBuf X, Xt, H1, H2, H1t, H2t, Y, dY, dYt, dH2, dH1, dH2t, dH1t, sse;
+    DevBuf X, H1, H2, dY, dH2, dH1;
+    DevBuf sse;                  // the loss's partial sums (one per CTA of the last layer)
+    double *sse_host = nullptr;  // their pinned copy
+    uint64_t sse_n = 0;
+    cudaEvent_t sse_ready = nullptr;
+
+    Mlp() = default;
+    Mlp(const Mlp &) = delete;
+    Mlp &operator=(const Mlp &) = delete;
+    ~Mlp();
 
     void init(uint32_t n_in, uint32_t n_hidden, uint32_t n_out, uint64_t seed);
-    // Y = MLP(X) for `batch` rows of FP32 X [batch][n_in] into FP32 Y (or the
-    // internal buffer when Y is null)
+    // Y = MLP(X) for `batch` rows of FP32 X [batch][n_in] into FP32 Y
     void forward(uint32_t batch, const float *X, float *Y);
     // gradients of the mean squared error against T at the current weights;
     // returns the loss
@@ -35,7 +43,9 @@ struct Mlp {
   private:
     void ensure(uint32_t batch);
     void refresh_bf16();
-    void transpose(const void *in, void *out, uint32_t rows, uint32_t cols);
+    void hidden(uint32_t batch, const float *X, bool split);
+    void backward(uint32_t batch, const float *X, const float *T);
+    double loss(uint32_t batch);
     static cudaStream_t S() { return ctx().stream; }
 };
 

@@ -87,7 +87,16 @@ namespace mm {
 // (+ bias), 2 BF16 ReLU(acc + bias), 3 BF16 acc masked by aux > 0.
 void gemm_bf16(uint64_t M, uint64_t N, uint64_t K, const void *A, const void *B, void *C,
                uint64_t ldc, int mode, const float *bias, const void *aux, uint64_t ld_aux,
-               cudaStream_t s);
+               cudaStream_t s, bool a_mn = false, bool b_mn = false, bool may_split = true);
+// a_mn / b_mn: A is stored transposed as [K][M], B as [K][N]. may_split: the
+// sum over K may be split between CTAs (another rounding of the same sums).
+// The last layer of a training pass: d = A B^T + bias - T, dY[M][N] = scale d
+// in BF16, and the sum of d^2 as one partial sum per CTA in sse; returns their
+// number, at most gemm_mse_parts.
+uint64_t gemm_mse_grad(uint64_t M, uint64_t N, uint64_t K, const void *A, const void *B, void *dY,
+                       const float *bias, const float *T, float scale, double *sse,
+                       cudaStream_t s);
+inline uint64_t gemm_mse_parts(uint64_t M, uint64_t N) { return (M / 128) * (N / 64); }
 }  // namespace mm
 
 void spmv_dot3(const DCsr &A, const double *sa, double *t, const double *s_, double *sc, int nv,

@@ -61,3 +61,34 @@ def test_gemm_rejects_bad_shapes(gpu):
     rc = gpu.lib().XAMG_b200_gemm_bf16(100, 128, 64, A.data_ptr(), A.data_ptr(), C.data_ptr(),
                                        128, 0, None, None, 0, None)
     assert rc == -2
+
+
+@pytest.mark.parametrize("M,N,K,mode", [(128, 256, 2368, 0),    # K split over a cluster, unevenly
+                                        (128, 1024, 1088, 2), (256, 384, 2048, 3),
+                                        (1280, 2048, 64, 1),    # one k-block, 256-wide tiles
+                                        (2176, 2304, 704, 0)])  # more tiles than SMs
+def test_gemm_tile_shapes(gpu, M, N, K, mode):
+    """The tile widths and K splits the launcher chooses between."""
+    got, ref, bound = run(gpu, M, N, K, mode, seed=M + K)
+    assert np.all(np.abs(got - ref) <= bound), np.abs(got - ref).max()
+
+
+def test_gemm_unaligned_bias_and_padded_rows(gpu):
+    """A bias that starts off a 16-byte boundary and rows of C wider than N."""
+    import torch
+    M, N, K, ldc = 128, 128, 1024, 136
+    g = torch.Generator().manual_seed(9)
+    A = torch.randn(M, K, generator=g).to(torch.bfloat16)
+    B = torch.randn(N, K, generator=g).to(torch.bfloat16)
+    bias = torch.randn(N + 1, generator=g)
+    Ad, Bd, bd = A.cuda(), B.cuda(), bias.cuda()
+    C = torch.full((M, ldc), 7.0, device="cuda")
+    gpu.call("XAMG_b200_gemm_bf16", M, N, K, Ad.data_ptr(), Bd.data_ptr(), C.data_ptr(), ldc, 0,
+             bd.data_ptr() + 4, None, 0, torch.cuda.current_stream().cuda_stream)
+    torch.cuda.synchronize()
+    ref = (A.double() @ B.double().T + bias[1:].double()).numpy()
+    bound = 2.0 * K * 2.0 ** -24 * (A.double().abs() @ B.double().abs().T).numpy() \
+        + 2.0 ** -23 * np.abs(ref)
+    got = C.cpu().double().numpy()
+    assert np.all(np.abs(got[:, :N] - ref) <= bound)
+    assert np.all(got[:, N:] == 7.0)

@@ -47,6 +47,46 @@ def test_gradients_against_oracle(gpu, n_in, h, n_out, B):
         assert np.abs(gb - rb).max() <= 1e-2 * np.abs(rb).max() + 1e-12
 
 
+@pytest.mark.parametrize("n_in,h,n_out,B", [(640, 384, 1152, 384), (256, 1024, 128, 640)])
+def test_gradients_of_several_tiles(gpu, n_in, h, n_out, B):
+    """Several tiles and K splits in every product, transposed operands included.
+    With B x h activations a pre-activation within the FP32 accumulation's error
+    of zero can fall on the other side of the ReLU than in the oracle: that
+    moves one sample's share of one row of a weight gradient, about
+    1 / sqrt(B h) of the block's norm (0.3 % here), so blocks are compared in
+    the 2-norm, 1 % allowing some ten of them."""
+    import torch
+    m = gpu.Mlp(n_in, h, n_out, seed=3)
+    p = m.params()
+    rng = np.random.default_rng(4)
+    X = rng.standard_normal((B, n_in)).astype(np.float32)
+    T = rng.standard_normal((B, n_out)).astype(np.float32)
+    Xd, Td = torch.from_numpy(X).cuda(), torch.from_numpy(T).cuda()
+    g, loss = m.gradients(Xd.data_ptr(), Td.data_ptr(), B)
+    gr, lr_ = MO.gradients(p.astype(np.float64), X.astype(np.float64), T.astype(np.float64),
+                           n_in, h, n_out)
+    assert abs(loss - lr_) <= 1e-3 * lr_
+    for gb, rb in zip(blocks(g, n_in, h, n_out), blocks(gr, n_in, h, n_out)):
+        assert np.linalg.norm(gb - rb) <= 1e-2 * np.linalg.norm(rb)
+
+
+def test_targets_off_a_16_byte_boundary(gpu):
+    """The loss gradient reads the targets in the last layer's epilogue: the
+    same loss and gradients for targets that start 4 bytes further."""
+    import torch
+    n_in, h, n_out, B = 256, 128, 256, 128
+    rng = np.random.default_rng(8)
+    X = torch.from_numpy(rng.standard_normal((B, n_in)).astype(np.float32)).cuda()
+    T = torch.from_numpy(rng.standard_normal(B * n_out).astype(np.float32)).cuda()
+    T1 = torch.empty(B * n_out + 1, dtype=torch.float32, device="cuda")
+    T1[1:] = T
+    torch.cuda.synchronize()
+    m = gpu.Mlp(n_in, h, n_out, seed=2)
+    g0, l0 = m.gradients(X.data_ptr(), T.data_ptr(), B)
+    g1, l1 = m.gradients(X.data_ptr(), T1.data_ptr() + 4, B)
+    assert l0 == l1 and g0.tobytes() == g1.tobytes()
+
+
 def test_training_reduces_the_loss(gpu):
     import torch
     n_in, h, n_out, B = 128, 256, 128, 512
