@@ -9,7 +9,9 @@
 
 #include <algorithm>
 #include <cmath>
+#include <cstring>
 #include <random>
+#include <thread>
 
 #include "device.h"
 #include "mlp.h"
@@ -183,6 +185,9 @@ void Mlp::ensure(uint32_t batch) {
 }
 
 Mlp::~Mlp() {
+    if (bounce) cudaFreeHost(bounce);
+    for (cudaStream_t c : copy_streams)
+        if (c) cudaStreamDestroy(c);
     if (sse_host) cudaFreeHost(sse_host);
     if (sse_ready) cudaEventDestroy(sse_ready);
 }
@@ -280,6 +285,47 @@ double Mlp::train_step(uint32_t batch, const float *Xf, const float *T, float lr
     return loss(batch);
 }
 
+// Device values to the caller's pageable memory. One cudaMemcpy moves 5 GB/s
+// there (the driver's single staging copy, and the first touch of the caller's
+// pages): 9.3 ms for the 47 MB of a 5,248-1,024 network. COPIERS threads each
+// take every COPIERS-th megabyte through a pinned buffer and a stream of their
+// own, so the transfers overlap the copies out.
+void Mlp::download(float *host, const float *dev, uint64_t count) {
+    constexpr uint64_t CHUNK = 1u << 20;
+    const uint64_t bytes = count * sizeof(float);
+    if (bytes < 4 * CHUNK) {
+        XG_CUDA(cudaMemcpy(host, dev, bytes, cudaMemcpyDeviceToHost));
+        return;
+    }
+    if (!bounce) XG_CUDA(cudaMallocHost((void **)&bounce, COPIERS * CHUNK));
+    for (cudaStream_t &c : copy_streams)
+        if (!c) XG_CUDA(cudaStreamCreateWithFlags(&c, cudaStreamNonBlocking));
+    const int device = ctx().device;
+    cudaError_t err[COPIERS];
+    auto copier = [&](int t) {
+        cudaError_t e = cudaSetDevice(device);
+        char *buf = bounce + (uint64_t)t * CHUNK;
+        for (uint64_t o = (uint64_t)t * CHUNK; o < bytes && e == cudaSuccess; o += COPIERS * CHUNK) {
+            const uint64_t len = std::min(CHUNK, bytes - o);
+            e = cudaMemcpyAsync(buf, (const char *)dev + o, len, cudaMemcpyDeviceToHost,
+                                copy_streams[t]);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(copy_streams[t]);
+            if (e == cudaSuccess) std::memcpy((char *)host + o, buf, len);
+        }
+        err[t] = e;
+    };
+    std::thread th[COPIERS - 1];
+    int started = 0;
+    try {
+        for (; started < COPIERS - 1; ++started) th[started] = std::thread(copier, started + 1);
+    } catch (...) {  // no more threads: this one takes their share
+    }
+    copier(0);
+    for (int t = 0; t < started; ++t) th[t].join();
+    for (int t = started + 1; t < COPIERS; ++t) copier(t);
+    for (cudaError_t e : err) XG_CUDA(e);
+}
+
 // Parameters in the order W1^T [h][in], b1, W2^T [h][h], b2, W3^T [out][h], b3.
 uint64_t Mlp::param_count() const {
     uint64_t n = 0;
@@ -297,7 +343,7 @@ void Mlp::copy_params(float *host, bool set, bool grads) {
             XG_CUDA(cudaMemcpy(w.p, host + off, nw * 4, cudaMemcpyHostToDevice));
             XG_CUDA(cudaMemcpy(b.p, host + off + nw, L.out * 4, cudaMemcpyHostToDevice));
         } else {
-            XG_CUDA(cudaMemcpy(host + off, w.p, nw * 4, cudaMemcpyDeviceToHost));
+            download(host + off, w.as<float>(), nw);
             XG_CUDA(cudaMemcpy(host + off + nw, b.p, L.out * 4, cudaMemcpyDeviceToHost));
         }
         off += nw + L.out;

@@ -23,6 +23,10 @@ struct Mlp {
     double *sse_host = nullptr;  // their pinned copy
     uint64_t sse_n = 0;
     cudaEvent_t sse_ready = nullptr;
+    // parameter read-back: pinned buffers and streams of its copying threads
+    static constexpr int COPIERS = 4;
+    char *bounce = nullptr;
+    cudaStream_t copy_streams[COPIERS] = {};
 
     Mlp() = default;
     Mlp(const Mlp &) = delete;
@@ -41,6 +45,7 @@ struct Mlp {
     void copy_params(float *host, bool set, bool grads);
 
   private:
+    void download(float *host, const float *dev, uint64_t count);
     void ensure(uint32_t batch);
     void refresh_bf16();
     void hidden(uint32_t batch, const float *X, bool split);
