@@ -17,7 +17,7 @@
 // row slot t/NV and right-hand side t%NV, so a tile covers 256/NV consecutive
 // rows and consecutive threads read consecutive x entries of a row. (The SpMV
 // runs these 256 canonical threads on 256/VK physical ones, each carrying VK
-// consecutive right-hand sides; see canon_finish.) Tiles are
+// consecutive right-hand sides; see canon_partial.) Tiles are
 // dealt round-robin to B = min(ntiles, 1184) blocks (8 per SM on 148 SMs).
 // Dot products are accumulated per thread in tile order, combined within a
 // warp by an xor butterfly (offsets 16..NV), across the 8 warps in warp
@@ -188,8 +188,11 @@ __device__ __forceinline__ void canon_finish(T (&acc)[NRED], const RedArgs &ra, 
 
 // ---------------------------------------------------------------------------
 // CSR SpMV with a compile-time epilogue.
-//   acc = epi.init(i,k); for j in row i: acc = acc + x[col[j]*NV+k] * val[j]
-//   epi.store(i, k, acc, terms[NRED])
+//   p = epi.pre<VK>(i, k0): the operands the row's epilogue needs
+//   y = epi.init(p); for j in row i: y = y + x[col[j]*NV+k] * val[j]
+//   epi.fin(i, k0, y, p, terms[VK][NRED])
+// for the VK right-hand sides a thread carries; init(i, k) and
+// store(i, k, y, terms) are the same for one right-hand side.
 // FX is the element type x is stored in; it is converted to F on load (the
 // fused form of vector::convert before a reduced-precision restriction).
 // ---------------------------------------------------------------------------
@@ -224,10 +227,10 @@ __device__ __forceinline__ uint64_t col_at(I c, uint64_t i) {
 }
 
 // Right-hand sides one SpMV thread carries: x[c*NV + k0 .. k0+VK-1] is
-// loaded with 16-byte (or 8-byte) vector loads, so a warp issues 1/VK of the
+// loaded with one vector load of up to 32 bytes, so a warp issues 1/VK of the
 // shared-memory reads of (column, value) and of the gather instructions that
 // a thread per right-hand side would. The canonical order does not change
-// (canon_finish).
+// (canon_partial).
 #ifndef XG_SPMV_VK64
 #define XG_SPMV_VK64 2  // FP64 x
 #endif
@@ -245,6 +248,15 @@ template <typename FX, int VK>
 __device__ __forceinline__ void ld_x(const FX *p, FX (&o)[VK]) {
     if constexpr (VK == 1) {
         o[0] = __ldg(p);
+    } else if constexpr (std::is_same<FX, double>::value && VK == 4) {
+        asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];"
+            : "=d"(o[0]), "=d"(o[1]), "=d"(o[2]), "=d"(o[3])
+            : "l"(p));
+    } else if constexpr (std::is_same<FX, float>::value && VK == 8) {
+        asm("ld.global.nc.v8.f32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+            : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]),
+              "=f"(o[7])
+            : "l"(p));
     } else if constexpr (std::is_same<FX, double>::value) {
 #pragma unroll
         for (int h = 0; h < VK; h += 2) {
@@ -268,18 +280,64 @@ __device__ __forceinline__ void ld_x(const FX *p, FX (&o)[VK]) {
     }
 }
 
-// Row accumulation, entry by entry in row order (the loop is unrolled so that
-// gathers of later entries can issue before earlier sums complete; the
-// additions stay in order). cl/vl point at the row's first entry.
-// Resident blocks the register budget is set for: 1024 threads an SM at 64
-// registers a thread, whatever the block size.
-template <int VK>
-constexpr int spmv_min_blocks() { return 4 * VK; }
+// VK consecutive values of a vector as one operand: 16-byte accesses where they
+// make up whole ones (the launcher checks the pointers' alignment).
+template <typename T, int VK>
+struct Vec {
+    T v[VK];
+};
+template <int VK, typename T>
+__device__ __forceinline__ Vec<T, VK> ldv(const T *p) {
+    Vec<T, VK> o;
+    if constexpr (VK * sizeof(T) % 16 == 0) {
+#pragma unroll
+        for (int h = 0; h < (int)(VK * sizeof(T) / 16); ++h)
+            reinterpret_cast<uint4 *>(o.v)[h] = reinterpret_cast<const uint4 *>(p)[h];
+    } else if constexpr (VK * sizeof(T) == 8) {
+        *reinterpret_cast<uint2 *>(o.v) = *reinterpret_cast<const uint2 *>(p);
+    } else {
+#pragma unroll
+        for (int v = 0; v < VK; ++v) o.v[v] = p[v];
+    }
+    return o;
+}
+template <int VK, typename T>
+__device__ __forceinline__ void stv(T *p, const Vec<T, VK> &o) {
+    if constexpr (VK * sizeof(T) % 16 == 0) {
+#pragma unroll
+        for (int h = 0; h < (int)(VK * sizeof(T) / 16); ++h)
+            reinterpret_cast<uint4 *>(p)[h] = reinterpret_cast<const uint4 *>(o.v)[h];
+    } else if constexpr (VK * sizeof(T) == 8) {
+        *reinterpret_cast<uint2 *>(p) = *reinterpret_cast<const uint2 *>(o.v);
+    } else {
+#pragma unroll
+        for (int v = 0; v < VK; ++v) p[v] = o.v[v];
+    }
+}
+inline bool aligned16(const void *p) { return (uintptr_t)p % 16 == 0; }
 
-#ifndef XG_SPMV_UNROLL
-#define XG_SPMV_UNROLL 4
-#endif
-constexpr int SPMV_UNROLL = XG_SPMV_UNROLL;
+// Register budget and gathers in flight, measured on the 27-point 128^3 matrix,
+// nv = 8 (us; gathers of up to 16 bytes, 1024 threads an SM and four entries at
+// a time with the leftover ones one by one, before):
+// * No dot products: 1024 threads an SM at 64 registers, four gathers of up to
+//   16 bytes at a time; with 32-byte gathers 640 threads at 102 registers, which
+//   hold four of them beside the epilogue's operands (at 64 registers the
+//   Chebyshev step spills). FP64 y = A x 272 -> 226, Chebyshev step 340 -> 248;
+//   BF16 values 150 -> 109 and 185 -> 137.
+// * Dot products: the canonical 1,184 blocks are eight an SM, so with four
+//   right-hand sides a thread 512 threads have 128 registers: eight 16-byte or
+//   six 32-byte gathers in flight. Three dots 340 -> 263 (FP32 x), 340 -> 269
+//   (FP64 x); one dot 285 -> 246.
+template <typename FX, int VK, int NRED>
+constexpr int spmv_min_blocks() {
+    if (NRED > 0) return VK > 1 ? 8 : 4;
+    return VK * sizeof(FX) >= 32 ? 5 * VK / 2 : 4 * VK;
+}
+template <typename FX, int VK, int NRED>
+constexpr int spmv_unroll() {
+    if (NRED > 0 && VK > 1) return VK < 4 ? 6 : sizeof(FX) == 8 ? 6 : 8;
+    return 4;
+}
 
 // A stored matrix value in the arithmetic type F: the value itself, or a
 // BF16 value widened exactly to float.
@@ -310,18 +368,45 @@ __device__ __forceinline__ uint32_t col_at32(I c, uint32_t i) {
         return (uint32_t)c;
 }
 
-template <typename F, typename FX, typename I, int NV, int VK, typename V = F>
+// Row accumulation, entry by entry in row order: U gathers issue before the
+// sums that use them, and a row's last few entries (27 = 6 x 4 + 3) issue
+// together too instead of one by one; the additions stay in order. cl/vl point at
+// the row's first entry.
+template <typename F, typename FX, typename I, int NV, int VK, int NRED, typename V = F>
 __device__ __forceinline__ void row_sum(F (&y)[VK], uint32_t len, uint64_t i, int k0, const I *cl,
                                         const V *vl, const FX *x, float vsc = 1.0f) {
     const uint32_t i32 = (uint32_t)i;
-#pragma unroll SPMV_UNROLL
-    for (uint32_t j = 0; j < len; ++j) {
-        const uint32_t c = col_at32<I>(cl[j], i32);
-        const F av = val_as<F, V>(vl[j], vsc);
-        FX xv[VK];
-        ld_x<FX, VK>(x + (c * (uint32_t)NV + (uint32_t)k0), xv);
+    constexpr int U = spmv_unroll<FX, VK, NRED>();
+    uint32_t j = 0;
+    for (; j + U <= len; j += U) {
+        F a[U];
+        FX xv[U][VK];
 #pragma unroll
-        for (int v = 0; v < VK; ++v) y[v] = add(y[v], mul((F)xv[v], av));
+        for (int q = 0; q < U; ++q) {
+            const uint32_t c = col_at32<I>(cl[j + q], i32);
+            a[q] = val_as<F, V>(vl[j + q], vsc);
+            ld_x<FX, VK>(x + (c * (uint32_t)NV + (uint32_t)k0), xv[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < U; ++q)
+#pragma unroll
+            for (int v = 0; v < VK; ++v) y[v] = add(y[v], mul((F)xv[q][v], a[q]));
+    }
+    if (j < len) {  // fewer than U left: the last entry stands in for the missing ones
+        F a[U];
+        FX xv[U][VK];
+#pragma unroll
+        for (int q = 0; q < U - 1; ++q) {
+            const uint32_t e = j + q < len ? j + q : len - 1;
+            const uint32_t c = col_at32<I>(cl[e], i32);
+            a[q] = val_as<F, V>(vl[e], vsc);
+            ld_x<FX, VK>(x + (c * (uint32_t)NV + (uint32_t)k0), xv[q]);
+        }
+#pragma unroll
+        for (int q = 0; q < U - 1; ++q)
+            if (j + q < len)
+#pragma unroll
+                for (int v = 0; v < VK; ++v) y[v] = add(y[v], mul((F)xv[q][v], a[q]));
     }
 }
 
@@ -432,7 +517,7 @@ __device__ __forceinline__ uint32_t stage_shift(const T *arr, uint32_t j0) {
 // successive tiles share columns in its SM's L1.
 template <typename F, typename FX, typename I, int NV, int VK, int NRED, class Epi,
           typename V = F>
-__global__ void __launch_bounds__(CT / VK, spmv_min_blocks<VK>())
+__global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED>())
     k_spmv(CsrArgs<F> A, const FX *__restrict__ x, Epi epi, RedArgs ra, uint32_t cap,
            uint32_t nbuf, uint32_t B, uint32_t run = 1, uint32_t stride = 0) {
     constexpr int G = NV / VK;
@@ -447,33 +532,62 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<VK>())
     const uint32_t *__restrict__ row = A.row;
     const I *__restrict__ col = (const I *)A.col;
     const V *__restrict__ val = (const V *)A.val;
-    const uint64_t n = A.n;
-    const uint64_t nnz = n ? row[n] : 0;
-    const uint64_t ntiles = (n + R - 1) / R;
-    // position after t in this physical block's sequence (ntiles: none);
-    // positions are tiles except in the plane walk below
-    auto next_tile = [&](uint64_t t) -> uint64_t {
+    const uint32_t n = (uint32_t)A.n;  // rows, tiles and elements fit in 32 bits (launcher)
+    const uint32_t ntiles = n / R + (n % R != 0);
+    // A position in this physical block's sequence of tiles (END: past it);
+    // positions are tiles except in the plane walk below. NRED == 0: `left`
+    // positions of the current run remain, this one included; NRED > 0: `left`
+    // is the canonical block.
+    constexpr uint32_t END = 0xFFFFFFFFu;
+    struct Pos {
+        uint32_t t, left;
+    };
+    auto after = [&](Pos p) -> Pos {
+        uint64_t t;
         if constexpr (NRED == 0) {
-            if ((t + 1) % run != 0 && t + 1 < ntiles) return t + 1;
-            const uint64_t q = (t / run + gridDim.x) * run;
-            return q < ntiles ? q : ntiles;
+            t = (uint64_t)p.t + 1;
+            if (p.left > 1) {
+                --p.left;
+            } else {
+                t += (uint64_t)(gridDim.x - 1) * run;
+                p.left = run;
+            }
+        } else {
+            t = (uint64_t)p.t + B;
+            if (t >= ntiles) {
+                p.left += gridDim.x;
+                t = p.left < B ? p.left : ntiles;
+            }
         }
-        if (t + B < ntiles) return t + B;
-        const uint64_t c = t % B + gridDim.x;
-        return c < B ? c : ntiles;
+        p.t = t < ntiles ? (uint32_t)t : END;
+        return p;
     };
     // Plane walk (no dot products, stride > 0): the blocks run through walk
     // positions u as above, position u being tile (u % M) * stride + u / M for
     // u < M * stride (M = ntiles / stride) and tile u after that: a
     // bijection, under which consecutive positions are tiles stride apart.
-    const uint64_t wM = (NRED == 0 && stride) ? ntiles / stride : 0;
-    const uint64_t wmain = wM * stride;
-    auto tile_at = [&](uint64_t u) -> uint64_t {
+    auto first_row = [&](uint32_t u) -> uint32_t {
         if constexpr (NRED == 0)
-            if (u < wmain) return (u % wM) * stride + u / wM;
-        return u;
+            if (stride) {
+                const uint32_t wM = ntiles / stride;
+                if (u < wM * stride) u = (u % wM) * stride + u / wM;
+            }
+        return u * R;
     };
-    const uint64_t first = NRED == 0 ? (uint64_t)blockIdx.x * run : (uint64_t)blockIdx.x;
+    // This thread's row of a tile: its index (n or more: none) and its entries.
+    // The row pointers are read a tile ahead of their use, so that neither
+    // the copy of the next tile nor the row sum waits for them.
+    struct Row {
+        uint32_t r0, j0, j1;
+    };
+    auto row_of = [&](uint32_t u) -> Row {
+        Row r;
+        r.r0 = first_row(u);
+        const uint32_t i = r.r0 + rt;
+        r.j0 = __ldg(&row[i < n ? i : n]);
+        r.j1 = __ldg(&row[i < n ? i + 1 : n]);
+        return r;
+    };
     F acc[VK][NR];
 #pragma unroll
     for (int v = 0; v < VK; ++v)
@@ -488,11 +602,10 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<VK>())
     __syncthreads();
     uint32_t n_issued = 0, n_used = 0;  // staged tiles issued (thread 0) / consumed
     bool timed_out = false;
-    // thread 0: copy tile t into the next buffer if it fits
-    auto issue = [&](uint64_t t) {
-        if (t >= ntiles) return;
-        const uint64_t a0 = t * R, a1 = a0 + R < n ? a0 + R : n;
-        const uint32_t j0 = row[a0], j1 = row[a1];
+    // first entry past a tile that starts at row r0
+    auto tile_end = [&](uint32_t r0) { return __ldg(&row[n - r0 > (uint32_t)R ? r0 + R : n]); };
+    // thread 0: copy a tile's entries into the next buffer if they fit
+    auto issue = [&](uint32_t j0, uint32_t j1) {
         if (j1 - j0 > CAP) return;
         unsigned char *buf = smem_raw + (size_t)(n_issued % nbuf) * BB;
         uint64_t *m = &mbar[n_issued % nbuf];
@@ -501,6 +614,7 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<VK>())
         V *vdst;
         const I *csrc;
         I *cdst;
+        const uint64_t nnz = __ldg(&row[n]);
         const uint32_t vb = stage_range<V>((V *)buf, val, nnz, j0, j1, vsrc, vdst);
         const uint32_t cb = stage_range<I>((I *)(buf + VB), col, nnz, j0, j1, csrc, cdst);
         mbar_arrive_expect(m, vb + cb);  // releases the plain-load writes above
@@ -508,17 +622,31 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<VK>())
         if (vb) bulk_g2s(vdst, vsrc, vb, m);
         if (cb) bulk_g2s(cdst, csrc, cb, m);
     };
-    if (threadIdx.x == 0) issue(tile_at(first));
-
-    for (uint64_t u = first; u < ntiles;) {
-        const uint64_t unext = next_tile(u);
-        const uint64_t tile = tile_at(u);
-        const uint64_t tnext = unext < ntiles ? tile_at(unext) : ntiles;
-        const uint64_t r0 = tile * R;
-        const uint64_t r1 = r0 + R < n ? r0 + R : n;
-        const uint32_t tj0 = __ldg(&row[r0]), tj1 = __ldg(&row[r1]);
-        bool staged = tj1 - tj0 <= CAP;
-        if (nbuf == 2 && threadIdx.x == 0) issue(tnext);
+    Pos at{NRED == 0 ? blockIdx.x * run : blockIdx.x, NRED == 0 ? run : blockIdx.x};
+    if (at.t >= ntiles) at.t = END;
+    Pos an = at;
+    Row cur{}, nxt{};
+    if (at.t != END) {
+        cur = row_of(at.t);
+        if (threadIdx.x == 0) issue(cur.j0, tile_end(cur.r0));  // thread 0 has the first row
+        an = after(at);
+        if (an.t != END) nxt = row_of(an.t);
+    }
+    while (at.t != END) {
+        const bool more = an.t != END;
+        if (nbuf == 2 && threadIdx.x == 0 && more) issue(nxt.j0, tile_end(nxt.r0));
+        Pos ann = an;
+        Row nn{};
+        if (more) {
+            ann = after(an);
+            if (ann.t != END) nn = row_of(ann.t);
+        }
+        const uint32_t i = cur.r0 + rt;
+        // the epilogue's operands are on their way while the row is summed
+        typename Epi::template Pre<VK> pre;
+        if (i < n) pre = epi.template pre<VK>(i, k0);
+        const uint32_t tj0 = __ldg(&row[cur.r0]);
+        bool staged = tile_end(cur.r0) - tj0 <= CAP;
         const V *sv = nullptr;
         const I *sc = nullptr;
         if (staged) {
@@ -531,26 +659,25 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<VK>())
             sc = (const I *)(buf + VB) + stage_shift<I>(col, tj0);
             staged = !timed_out;
         }
-        const uint64_t i = r0 + rt;
         if (i < n) {
             F y[VK];
-#pragma unroll
-            for (int v = 0; v < VK; ++v) y[v] = epi.init(i, k0 + v);
-            const uint32_t j0 = __ldg(&row[i]), j1 = __ldg(&row[i + 1]);
+            epi.template init<VK>(y, pre);
+            const uint32_t len = cur.j1 - cur.j0, o = cur.j0 - tj0;
             if (staged)
-                row_sum<F, FX, I, NV, VK, V>(y, j1 - j0, i, k0, sc + (j0 - tj0), sv + (j0 - tj0),
-                                             x, A.vscale);
+                row_sum<F, FX, I, NV, VK, NRED, V>(y, len, i, k0, sc + o, sv + o, x, A.vscale);
             else
-                row_sum<F, FX, I, NV, VK, V>(y, j1 - j0, i, k0, col + j0, val + j0, x, A.vscale);
-#pragma unroll
-            for (int v = 0; v < VK; ++v) epi.store(i, k0 + v, y[v], acc[v]);
+                row_sum<F, FX, I, NV, VK, NRED, V>(y, len, i, k0, col + cur.j0, val + cur.j0, x,
+                                             A.vscale);
+            epi.template fin<VK>(i, k0, y, pre, acc);
         }
         __syncthreads();  // every reader is done with this tile's buffer
-        if (nbuf == 1 && threadIdx.x == 0) issue(tnext);
+        if (nbuf == 1 && threadIdx.x == 0 && more) issue(nxt.j0, tile_end(nxt.r0));
         if constexpr (NRED > 0)
-            if (tnext == ntiles || tnext % B != tile % B)
-                canon_partial<F, NV, NRED, VK>(acc, ra, (uint32_t)(tile % B));
-        u = unext;
+            if (!more || an.left != at.left) canon_partial<F, NV, NRED, VK>(acc, ra, at.left);
+        at = an;
+        an = ann;
+        cur = nxt;
+        nxt = nn;
     }
     if (timed_out) {
         atomicOr(ra.flag, 1u);
@@ -563,49 +690,85 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<VK>())
 
 // Warp-per-row SpMV for matrices with few rows (the coarse levels and their
 // transfers), where k_spmv's time is one thread's chain of gathers down a
-// whole row. A warp takes one row at a time: its lanes gather the products
-// of 32/NV entries at once (lane = entry slot * NV + right-hand side), each
+// whole row. A warp takes one row at a time: its lanes read up to 32 entries
+// (one each, coalesced), then gather the products of 32/NV entries at once
+// (lane = entry slot * NV + right-hand side, the entry by shuffle), each
 // product rounded on its own (mul(x, a), as row_sum rounds it), into a
 // shared-memory chunk of WCH entries; then lane k < NV adds the chunk's
 // products to its sum in entry order. So every output element is the same
 // sequence of separately rounded products and sums as in k_spmv, while a
-// row's gathers are in flight together.
+// row's gathers are in flight together. The next entries, the next row's
+// pointers and the epilogue's operands are on their way meanwhile.
 constexpr int WT = 256;  // threads per block (8 warps)
 template <int NV>
 constexpr int wide_chunk() { return 512 / NV; }  // entries per warp-chunk
 template <typename F, typename FX, typename I, int NV, class Epi, typename V = F>
 __global__ void __launch_bounds__(WT) k_spmv_wide(CsrArgs<F> A, const FX *__restrict__ x, Epi epi) {
-    constexpr int E = NV >= 32 ? 1 : 32 / NV;  // entries a warp gathers per round
+    constexpr int E = 32 / NV;  // entries a warp gathers per round
     constexpr int CH = wide_chunk<NV>();
+    constexpr int GE = CH < 32 ? CH : 32;  // entries read at once, one a lane
     __shared__ F prod[WT / 32][CH * NV];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int k = lane % NV, es = lane / NV;  // es < E for NV <= 32
+    const int k = lane % NV, es = lane / NV;
     const uint32_t *__restrict__ row = A.row;
     const I *__restrict__ col = (const I *)A.col;
     const V *__restrict__ val = (const V *)A.val;
     F *pw = prod[warp];
     const uint64_t nw = (uint64_t)gridDim.x * (WT / 32);
-    for (uint64_t i = (uint64_t)blockIdx.x * (WT / 32) + warp; i < A.n; i += nw) {
-        const uint32_t j0 = __ldg(&row[i]), j1 = __ldg(&row[i + 1]);
+    uint64_t i = (uint64_t)blockIdx.x * (WT / 32) + warp;
+    uint32_t j0 = 0, j1 = 0;
+    if (i < A.n) {
+        j0 = __ldg(&row[i]);
+        j1 = __ldg(&row[i + 1]);
+    }
+    for (; i < A.n; i += nw) {
         const uint32_t i32 = (uint32_t)i;
-        F y = k < NV && lane < NV ? epi.init(i, k) : F(0);
+        typename Epi::template Pre<1> pre;
+        F y[1] = {F(0)};
+        uint32_t nj0 = 0, nj1 = 0;
+        uint32_t cn = 0;  // entry j0 + lane of the group to come
+        F vn = F(0);
+        if (lane < GE && j0 + lane < j1) {
+            cn = col_at32<I>(__ldg(&col[j0 + lane]), i32);
+            vn = val_as<F, V>(__ldg(&val[j0 + lane]), A.vscale);
+        }
+        if (lane < NV) pre = epi.template pre<1>(i32, lane);
+        if (i + nw < A.n) {
+            nj0 = __ldg(&row[i + nw]);
+            nj1 = __ldg(&row[i + nw + 1]);
+        }
+        if (lane < NV) epi.template init<1>(y, pre);
         for (uint32_t c0 = j0; c0 < j1; c0 += CH) {
             const uint32_t len = j1 - c0 < (uint32_t)CH ? j1 - c0 : (uint32_t)CH;
-#pragma unroll 4
-            for (uint32_t e = es; e < len; e += E) {
-                const uint32_t c = col_at32<I>(__ldg(&col[c0 + e]), i32);
-                const F av = val_as<F, V>(__ldg(&val[c0 + e]), A.vscale);
-                pw[e * NV + k] = mul((F)__ldg(&x[c * (uint32_t)NV + (uint32_t)k]), av);
+            for (uint32_t g0 = 0; g0 < len; g0 += GE) {
+                const uint32_t c = cn;
+                const F av = vn;
+                const uint32_t jn = c0 + g0 + GE + lane;
+                if (lane < GE && jn < j1) {
+                    cn = col_at32<I>(__ldg(&col[jn]), i32);
+                    vn = val_as<F, V>(__ldg(&val[jn]), A.vscale);
+                }
+#pragma unroll 8
+                for (int r = 0; r < GE / E; ++r) {
+                    const int e = r * E + es;
+                    const uint32_t ce = __shfl_sync(0xffffffffu, c, e);
+                    const F ae = __shfl_sync(0xffffffffu, av, e);
+                    if (g0 + e < len)
+                        pw[(g0 + e) * NV + k] =
+                            mul((F)__ldg(&x[ce * (uint32_t)NV + (uint32_t)k]), ae);
+                }
             }
             __syncwarp();
             if (lane < NV) {
 #pragma unroll 8
-                for (uint32_t e = 0; e < len; ++e) y = add(y, pw[e * NV + lane]);
+                for (uint32_t e = 0; e < len; ++e) y[0] = add(y[0], pw[e * NV + lane]);
             }
             __syncwarp();
         }
-        F none[1] = {F(0)};
-        if (lane < NV) epi.store(i, lane, y, none);
+        F none[1][1] = {{F(0)}};
+        if (lane < NV) epi.template fin<1>(i32, lane, y, pre, none);
+        j0 = nj0;
+        j1 = nj1;
     }
 }
 
@@ -668,37 +831,102 @@ struct NoFin {
     __device__ void operator()(int, const T *) const {}
 };
 
+// What every SpMV epilogue shares: a row sum that starts from zero, and the
+// one-right-hand-side forms written with the vector ones. D is the epilogue,
+// F its arithmetic type. Elements are indexed in 32 bits (the launchers check
+// that they fit).
+template <class D, typename F>
+struct EpiBase {
+    __device__ F init(uint64_t, int) const { return F(0); }
+    template <int VK, class P>
+    __device__ void init(F (&y)[VK], const P &) const {
+#pragma unroll
+        for (int v = 0; v < VK; ++v) y[v] = F(0);
+    }
+    template <int NR>
+    __device__ void store(uint64_t i, int k, F v, F (&acc)[NR]) const {
+        const D &d = static_cast<const D &>(*this);
+        F y[1] = {v};
+        d.template fin<1>((uint32_t)i, k, y, d.template pre<1>((uint32_t)i, k), reinterpret_cast<F(&)[1][NR]>(acc));
+    }
+};
+
 // y = A x  (csr_matvec.inl:213-231)
 template <typename F, int NV>
-struct EStore : NoFin {
+struct EStore : EpiBase<EStore<F, NV>, F>, NoFin {
     F *y;
-    __device__ F init(uint64_t, int) const { return F(0); }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, F v, F (&)[NR]) const { y[i * NV + k] = v; }
+    __host__ __device__ explicit EStore(F *y_) : y(y_) {}
+    bool aligned() const { return aligned16(y); }
+    template <int VK>
+    struct Pre {};
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t, int) const { return {}; }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const F (&s)[VK], const Pre<VK> &,
+                        F (&)[VK][NR]) const {
+        Vec<F, VK> o;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) o.v[v] = s[v];
+        stv<VK>(y + (i * NV + k0), o);
+    }
 };
 
 // y += A x  (csr_matvec.inl:106-120: accumulate directly into y)
 template <typename F, int NV>
 struct EAxpy : NoFin {
     F *y;
+    __host__ __device__ explicit EAxpy(F *y_) : y(y_) {}
+    bool aligned() const { return aligned16(y); }
+    template <int VK>
+    struct Pre {
+        Vec<F, VK> y;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const { return {ldv<VK>(y + (i * NV + k0))}; }
     __device__ F init(uint64_t i, int k) const { return y[i * NV + k]; }
+    template <int VK>
+    __device__ void init(F (&s)[VK], const Pre<VK> &p) const {
+#pragma unroll
+        for (int v = 0; v < VK; ++v) s[v] = p.y.v[v];
+    }
     template <int NR>
     __device__ void store(uint64_t i, int k, F v, F (&)[NR]) const { y[i * NV + k] = v; }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const F (&s)[VK], const Pre<VK> &,
+                        F (&)[VK][NR]) const {
+        Vec<F, VK> o;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) o.v[v] = s[v];
+        stv<VK>(y + (i * NV + k0), o);
+    }
 };
 
 // r = 1*b + (-1)*(A x)  (solver.h:249-250: Ax_y then axpby(1, b, -1, r)),
 // optionally with (r, r) (vector_norm, blas.inl:537-555).
 template <typename F, int NV, bool NORM>
-struct EResid {
+struct EResid : EpiBase<EResid<F, NV, NORM>, F> {
     F *r;
     const F *b;
     double *out;  // NORM: sums land here (nv values)
-    __device__ F init(uint64_t, int) const { return F(0); }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, F v, F (&acc)[NR]) const {
-        const F rv = add(mul(F(1), b[i * NV + k]), mul(F(-1), v));
-        r[i * NV + k] = rv;
-        if constexpr (NORM) acc[0] = add(acc[0], mul(rv, rv));
+    EResid(F *r_, const F *b_, double *out_) : r(r_), b(b_), out(out_) {}
+    bool aligned() const { return aligned16(r) && aligned16(b); }
+    template <int VK>
+    struct Pre {
+        Vec<F, VK> b;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const { return {ldv<VK>(b + (i * NV + k0))}; }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const F (&s)[VK], const Pre<VK> &p,
+                        F (&acc)[VK][NR]) const {
+        Vec<F, VK> o;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            const F rv = add(mul(F(1), p.b.v[v]), mul(F(-1), s[v]));
+            o.v[v] = rv;
+            if constexpr (NORM) acc[v][0] = add(acc[v][0], mul(rv, rv));
+        }
+        stv<VK>(r + (i * NV + k0), o);
     }
     __device__ void operator()(int k, const F *s) const {
         if constexpr (NORM) out[k] = (double)s[0];
@@ -707,21 +935,39 @@ struct EResid {
 
 // merged_bicgstab_group1 after r0 = A x (blas_merged_bicgstab.inl:60-72):
 // r0 = b - r0; rho0 += r0*r0; p = r = r0. The finaliser also copies
-// rho0 into rho (merged_bicgstab.inl:119).
+// rho0 into rho (merged_bicgstab.inl:119). Element by element: the kernel-level
+// entry point passes a caller's vectors, whatever their alignment.
 template <int NV>
-struct EGroup1 {
+struct EGroup1 : EpiBase<EGroup1<NV>, double> {
     double *r0, *p, *r;
     const double *b;
     double *sc;
-    __device__ double init(uint64_t, int) const { return 0.0; }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, double v, double (&acc)[NR]) const {
-        const uint64_t e = i * NV + k;
-        const double rv = sub(b[e], v);
-        r0[e] = rv;
-        p[e] = rv;
-        r[e] = rv;
-        acc[0] = add(acc[0], mul(rv, rv));
+    EGroup1(double *r0_, double *p_, double *r_, const double *b_, double *sc_)
+        : r0(r0_), p(p_), r(r_), b(b_), sc(sc_) {}
+    bool aligned() const { return true; }
+    template <int VK>
+    struct Pre {
+        double b[VK];
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const {
+        Pre<VK> o;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) o.b[v] = b[i * NV + k0 + v];
+        return o;
+    }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const double (&s)[VK], const Pre<VK> &q,
+                        double (&acc)[VK][NR]) const {
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            const uint32_t e = i * NV + k0 + v;
+            const double rv = sub(q.b[v], s[v]);
+            r0[e] = rv;
+            p[e] = rv;
+            r[e] = rv;
+            acc[v][0] = add(acc[v][0], mul(rv, rv));
+        }
     }
     __device__ void operator()(int k, const double *s) const {
         sc[SC_RHO0 * SC_STRIDE + k] = s[0];
@@ -732,16 +978,29 @@ struct EGroup1 {
 // v = A p_ ; scal1 = (v, r0) ; alpha = rho / scal1
 // (merged_pbicgstab.inl:140-155)
 template <int NV>
-struct EDotAlpha {
+struct EDotAlpha : EpiBase<EDotAlpha<NV>, double> {
     double *v;
     const double *r0;
     double *sc;
-    __device__ double init(uint64_t, int) const { return 0.0; }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, double y, double (&acc)[NR]) const {
-        const uint64_t e = i * NV + k;
-        v[e] = y;
-        acc[0] = add(acc[0], mul(y, r0[e]));
+    __host__ __device__ EDotAlpha(double *v_, const double *r0_, double *sc_)
+        : v(v_), r0(r0_), sc(sc_) {}
+    bool aligned() const { return aligned16(v) && aligned16(r0); }
+    template <int VK>
+    struct Pre {
+        Vec<double, VK> r0;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const { return {ldv<VK>(r0 + (i * NV + k0))}; }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const double (&s)[VK], const Pre<VK> &p,
+                        double (&acc)[VK][NR]) const {
+        Vec<double, VK> o;
+#pragma unroll
+        for (int w = 0; w < VK; ++w) {
+            o.v[w] = s[w];
+            acc[w][0] = add(acc[w][0], mul(s[w], p.r0.v[w]));
+        }
+        stv<VK>(v + (i * NV + k0), o);
     }
     __device__ void operator()(int k, const double *s) const {
         sc[SC_SCAL1 * SC_STRIDE + k] = s[0];
@@ -753,19 +1012,31 @@ struct EDotAlpha {
 // res = theta - omega*phi; alpha_c = iconv*alpha; omega_c = iconv*omega
 // (merged_pbicgstab.inl:168-192)
 template <int NV>
-struct EDot3 {
+struct EDot3 : EpiBase<EDot3<NV>, double> {
     double *t;
     const double *s;
     double *sc;
-    __device__ double init(uint64_t, int) const { return 0.0; }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, double y, double (&acc)[NR]) const {
-        const uint64_t e = i * NV + k;
-        t[e] = y;
-        const double sv = s[e];
-        acc[0] = add(acc[0], mul(y, sv));
-        acc[1] = add(acc[1], mul(y, y));
-        acc[2] = add(acc[2], mul(sv, sv));
+    __host__ __device__ EDot3(double *t_, const double *s_, double *sc_) : t(t_), s(s_), sc(sc_) {}
+    bool aligned() const { return aligned16(t) && aligned16(s); }
+    template <int VK>
+    struct Pre {
+        Vec<double, VK> s;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const { return {ldv<VK>(s + (i * NV + k0))}; }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const double (&y)[VK], const Pre<VK> &p,
+                        double (&acc)[VK][NR]) const {
+        Vec<double, VK> o;
+#pragma unroll
+        for (int w = 0; w < VK; ++w) {
+            const double sv = p.s.v[w];
+            o.v[w] = y[w];
+            acc[w][0] = add(acc[w][0], mul(y[w], sv));
+            acc[w][1] = add(acc[w][1], mul(y[w], y[w]));
+            acc[w][2] = add(acc[w][2], mul(sv, sv));
+        }
+        stv<VK>(t + (i * NV + k0), o);
     }
     __device__ void operator()(int k, const double *s3) const {
         double *S = sc;
@@ -787,15 +1058,30 @@ struct EDot3 {
 // One Jacobi sweep with x not zero (blas_merged_jacobi.inl:74-80):
 // x_out = x_in + relax*d*(b - A x_in)
 template <typename F, int NV>
-struct EJacobi : NoFin {
+struct EJacobi : EpiBase<EJacobi<F, NV>, F>, NoFin {
     F *xout;
     const F *xin, *b, *d;
     F relax;
-    __device__ F init(uint64_t, int) const { return F(0); }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, F v, F (&)[NR]) const {
-        const uint64_t e = i * NV + k;
-        xout[e] = add(xin[e], mul(mul(relax, d[i]), sub(b[e], v)));
+    __host__ __device__ EJacobi(F *xout_, const F *xin_, const F *b_, const F *d_, F relax_)
+        : xout(xout_), xin(xin_), b(b_), d(d_), relax(relax_) {}
+    bool aligned() const { return aligned16(xout) && aligned16(xin) && aligned16(b); }
+    template <int VK>
+    struct Pre {
+        Vec<F, VK> x, b;
+        F d;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const {
+        return {ldv<VK>(xin + (i * NV + k0)), ldv<VK>(b + (i * NV + k0)), d[i]};
+    }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const F (&s)[VK], const Pre<VK> &p,
+                        F (&)[VK][NR]) const {
+        Vec<F, VK> o;
+#pragma unroll
+        for (int v = 0; v < VK; ++v)
+            o.v[v] = add(p.x.v[v], mul(mul(relax, p.d), sub(p.b.v[v], s[v])));
+        stv<VK>(xout + (i * NV + k0), o);
     }
 };
 
@@ -803,26 +1089,41 @@ struct EJacobi : NoFin {
 // r = b - A x; r := r*isd; t1 = c_top * r; t1 := t1*isd (input of the next
 // SpMV). x_zero: r = 1*b without the SpMV (used by k_rows through elem()).
 template <typename F, int NV>
-struct ECheby0 : NoFin {
+struct ECheby0 : EpiBase<ECheby0<F, NV>, F>, NoFin {
     F *rs, *t1s;
     const F *b, *isd;
     F c;
-    __device__ F init(uint64_t, int) const { return F(0); }
-    __device__ void finish(uint64_t i, int k, F r) const {
-        const uint64_t e = i * NV + k;
-        const F d = isd[i];
-        const F rr = mul(r, d);
-        rs[e] = rr;
-        t1s[e] = mul(mul(c, rr), d);
+    ECheby0(F *rs_, F *t1s_, const F *b_, const F *isd_, F c_)
+        : rs(rs_), t1s(t1s_), b(b_), isd(isd_), c(c_) {}
+    bool aligned() const { return aligned16(rs) && aligned16(t1s) && aligned16(b); }
+    template <int VK>
+    struct Pre {
+        Vec<F, VK> b;
+        F d;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const {
+        return {ldv<VK>(b + (i * NV + k0)), isd[i]};
     }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, F v, F (&)[NR]) const {
-        const uint64_t e = i * NV + k;
-        finish(i, k, add(mul(F(1), b[e]), mul(F(-1), v)));
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const F (&s)[VK], const Pre<VK> &p,
+                        F (&)[VK][NR]) const {
+        Vec<F, VK> rr, t1;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            rr.v[v] = mul(add(mul(F(1), p.b.v[v]), mul(F(-1), s[v])), p.d);
+            t1.v[v] = mul(mul(c, rr.v[v]), p.d);
+        }
+        stv<VK>(rs + (i * NV + k0), rr);
+        stv<VK>(t1s + (i * NV + k0), t1);
     }
     template <int NR>
     __device__ void elem(uint64_t i, int k, F (&)[NR]) const {
-        finish(i, k, mul(F(1), b[i * NV + k]));
+        const uint64_t e = i * NV + k;
+        const F d = isd[i];
+        const F rr = mul(mul(F(1), b[e]), d);
+        rs[e] = rr;
+        t1s[e] = mul(mul(c, rr), d);
     }
 };
 
@@ -830,25 +1131,44 @@ struct ECheby0 : NoFin {
 // t2 = A t1s; t2 := t2*isd; t1 = c_i*rs + 1*t2; then either t1s_out = t1*isd
 // (more steps) or x = 1*(t1*isd) + 1*x (last step; x_zero: x = 1*(t1*isd)).
 template <typename F, int NV>
-struct ECheby1 : NoFin {
+struct ECheby1 : EpiBase<ECheby1<F, NV>, F>, NoFin {
     F *out;  // next t1s, or x on the last step
     const F *rs, *isd;
     F c;
     int last, x_zero;
-    __device__ F init(uint64_t, int) const { return F(0); }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, F v, F (&)[NR]) const {
-        const uint64_t e = i * NV + k;
-        const F d = isd[i];
-        const F t2 = mul(v, d);
-        const F t1 = add(mul(c, rs[e]), mul(F(1), t2));
-        const F t1d = mul(t1, d);
-        if (!last)
-            out[e] = t1d;
-        else if (x_zero)
-            out[e] = mul(F(1), t1d);
-        else
-            out[e] = add(mul(F(1), t1d), mul(F(1), out[e]));
+    ECheby1(F *out_, const F *rs_, const F *isd_, F c_, int last_, int x_zero_)
+        : out(out_), rs(rs_), isd(isd_), c(c_), last(last_), x_zero(x_zero_) {}
+    bool aligned() const { return aligned16(out) && aligned16(rs); }
+    template <int VK>
+    struct Pre {
+        Vec<F, VK> rs, x;
+        F d;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const {
+        Pre<VK> p;
+        p.rs = ldv<VK>(rs + (i * NV + k0));
+        if (last && !x_zero) p.x = ldv<VK>(out + (i * NV + k0));
+        p.d = isd[i];
+        return p;
+    }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const F (&s)[VK], const Pre<VK> &p,
+                        F (&)[VK][NR]) const {
+        Vec<F, VK> o;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            const F t2 = mul(s[v], p.d);
+            const F t1 = add(mul(c, p.rs.v[v]), mul(F(1), t2));
+            const F t1d = mul(t1, p.d);
+            if (!last)
+                o.v[v] = t1d;
+            else if (x_zero)
+                o.v[v] = mul(F(1), t1d);
+            else
+                o.v[v] = add(mul(F(1), t1d), mul(F(1), p.x.v[v]));
+        }
+        stv<VK>(out + (i * NV + k0), o);
     }
 };
 
@@ -856,15 +1176,31 @@ struct ECheby1 : NoFin {
 // accumulated in float, converted to double, then x = 1*t + 1*x
 // (x_zero: x = 1*t, the ax_y branch of axpby).
 template <int NV>
-struct EProlongMixed : NoFin {
+struct EProlongMixed : EpiBase<EProlongMixed<NV>, float>, NoFin {
     double *x;
     int x_zero;
-    __device__ float init(uint64_t, int) const { return 0.0f; }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, float v, float (&)[NR]) const {
-        const uint64_t e = i * NV + k;
-        const double t = (double)v;
-        x[e] = x_zero ? mul(1.0, t) : add(mul(1.0, t), mul(1.0, x[e]));
+    EProlongMixed(double *x_, int x_zero_) : x(x_), x_zero(x_zero_) {}
+    bool aligned() const { return aligned16(x); }
+    template <int VK>
+    struct Pre {
+        Vec<double, VK> x;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const {
+        Pre<VK> p;
+        if (!x_zero) p.x = ldv<VK>(x + (i * NV + k0));
+        return p;
+    }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const float (&s)[VK], const Pre<VK> &p,
+                        float (&)[VK][NR]) const {
+        Vec<double, VK> o;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            const double t = (double)s[v];
+            o.v[v] = x_zero ? mul(1.0, t) : add(mul(1.0, t), mul(1.0, p.x.v[v]));
+        }
+        stv<VK>(x + (i * NV + k0), o);
     }
 };
 
@@ -992,16 +1328,28 @@ using OpXUpdate = OpXUpdateT<double>;
 // alpha = scal1 / scal2, alpha_conv = iconv * alpha, then alpha = -1 * alpha
 // (kept in SC_NSCAL). scal1 = (r, z) is the previous (r, z) (EPcgDots).
 template <int NV>
-struct EPcgAp {
+struct EPcgAp : EpiBase<EPcgAp<NV>, double> {
     double *Ap;
     const double *p;
     double *sc;
-    __device__ double init(uint64_t, int) const { return 0.0; }
-    template <int NR>
-    __device__ void store(uint64_t i, int k, double y, double (&acc)[NR]) const {
-        const uint64_t e = i * NV + k;
-        Ap[e] = y;
-        acc[0] = add(acc[0], mul(p[e], y));
+    EPcgAp(double *Ap_, const double *p_, double *sc_) : Ap(Ap_), p(p_), sc(sc_) {}
+    bool aligned() const { return aligned16(Ap) && aligned16(p); }
+    template <int VK>
+    struct Pre {
+        Vec<double, VK> p;
+    };
+    template <int VK>
+    __device__ Pre<VK> pre(uint32_t i, int k0) const { return {ldv<VK>(p + (i * NV + k0))}; }
+    template <int VK, int NR>
+    __device__ void fin(uint32_t i, int k0, const double (&y)[VK], const Pre<VK> &q,
+                        double (&acc)[VK][NR]) const {
+        Vec<double, VK> o;
+#pragma unroll
+        for (int w = 0; w < VK; ++w) {
+            o.v[w] = y[w];
+            acc[w][0] = add(acc[w][0], mul(q.p.v[w], y[w]));
+        }
+        stv<VK>(Ap + (i * NV + k0), o);
     }
     __device__ void operator()(int k, const double *s) const {
         double *S = sc;
@@ -1312,40 +1660,6 @@ __global__ void __launch_bounds__(CT)
     for (uint64_t i = r1; i-- > r0;) upd(i);
 }
 
-// Dense y = A_inv b (dense_matvec.inl:109-117): thread (i, k) accumulates
-// over j in order. The inverse is stored column by column (element (i, j)
-// at j*n + i). A block of DT threads holds DT/NV consecutive rows; it copies
-// chunks of DJ columns of its rows and the matching DJ rows of x into shared
-// memory with coalesced loads, then every thread runs its sum over the chunk
-// from shared memory, so the sequential sums wait on shared memory rather
-// than on L2.
-constexpr int DT = 64;
-constexpr int DJ = 64;
-template <typename F, int NV>
-__global__ void __launch_bounds__(DT)
-    k_dense(const F *__restrict__ a, uint64_t n, const F *__restrict__ x, F *__restrict__ y) {
-    constexpr int RB = DT / NV;  // rows a block
-    __shared__ F xs[DJ * NV];
-    __shared__ F as[DJ * RB];
-    const int r = threadIdx.x / NV, k = threadIdx.x % NV;
-    const uint64_t i0 = (uint64_t)blockIdx.x * RB;
-    const uint64_t i = i0 + r;
-    F acc = F(0);
-    for (uint64_t j0 = 0; j0 < n; j0 += DJ) {
-        const int jc = (int)(n - j0 < (uint64_t)DJ ? n - j0 : (uint64_t)DJ);
-        __syncthreads();  // the previous chunk is consumed
-        for (int t = threadIdx.x; t < jc * NV; t += DT) xs[t] = __ldg(&x[j0 * NV + t]);
-        for (int t = threadIdx.x; t < jc * RB; t += DT) {
-            const int jj = t / RB, rr = t % RB;
-            as[t] = i0 + rr < n ? __ldg(&a[(j0 + jj) * n + i0 + rr]) : F(0);
-        }
-        __syncthreads();
-        if (i < n)
-            for (int jj = 0; jj < jc; ++jj) acc = add(acc, mul(as[jj * RB + r], xs[jj * NV + k]));
-    }
-    if (i < n) y[i * NV + k] = acc;
-}
-
 // --- persistent preconditioned BiCGStab ----------------------------------------
 // Grid barrier with a bounded wait: every block of a cooperative launch
 // arrives on one 64-bit counter (zero at the launch's start; round r ends when
@@ -1538,7 +1852,7 @@ __global__ void __launch_bounds__(CT, 1) k_pbicgstab_persist(CsrArgs<double> A, 
         for (int j = 2; j <= m; ++j) {
             if (!sync()) return false;
             double *o = tgt(j);
-            const EJacobi<double, NV> ej{{}, o, cur, in, P.d, P.relax};
+            const EJacobi<double, NV> ej(o, cur, in, P.d, P.relax);
             double none[1];
             each([&](uint64_t i, uint64_t) { ej.store(i, kk, rowsum(cur, i), none); });
             cur = o;
@@ -1563,7 +1877,7 @@ __global__ void __launch_bounds__(CT, 1) k_pbicgstab_persist(CsrArgs<double> A, 
         if (!(ok = precond(P.pa, P.p))) break;
         if (!(ok = sync())) break;
         {   // v = A p_; alpha = rho / (v, r0)
-            const EDotAlpha<NV> ea{P.v, P.r0, SCS};
+            const EDotAlpha<NV> ea(P.v, P.r0, SCS);
             double acc[1][1] = {{0.0}};
             if (!(ok = reduce_each(
                       acc,
@@ -1580,7 +1894,7 @@ __global__ void __launch_bounds__(CT, 1) k_pbicgstab_persist(CsrArgs<double> A, 
         if (!(ok = precond(P.sa, P.s))) break;
         if (!(ok = sync())) break;
         {   // t = A s_; omega, res
-            const EDot3<NV> e3{P.t, P.s, SCS};
+            const EDot3<NV> e3(P.t, P.s, SCS);
             double acc[1][3] = {{0.0, 0.0, 0.0}};
             if (!(ok = reduce_each(
                       acc,

@@ -1,5 +1,6 @@
 // Launchers of the block smoother (hybrid symmetric Gauss-Seidel) and the dense
 // coarse solve.
+#include "dense.cuh"
 #include "hsgs.cuh"
 #include "spmv_launch.cuh"
 
@@ -71,8 +72,10 @@ void dense_apply(const F *a, uint64_t n, const F *x, F *y, int nv, cudaStream_t 
     if (n == 0) return;
     dispatch_nv(nv, [&](auto nvc) {
         constexpr int NV = decltype(nvc)::value;
-        constexpr uint64_t RB = k::DT / NV;
-        k::k_dense<F, NV><<<(unsigned)((n + RB - 1) / RB), k::DT, 0, s>>>(a, n, x, y);
+        constexpr uint64_t RB = k::dense_rows<F, NV>();
+        const uint32_t chunk = (uint32_t)std::min<uint64_t>(n, k::dense_chunk<F, NV>());
+        k::k_dense<F, NV><<<(unsigned)((n + RB - 1) / RB), k::DT, chunk * (NV + RB) * sizeof(F),
+                            s>>>(a, n, x, y, chunk);
         XG_CUDA(cudaGetLastError());
         ++g_kernel_launches;
     });

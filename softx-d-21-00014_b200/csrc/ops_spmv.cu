@@ -14,9 +14,9 @@ template <typename F>
 void spmv(const DCsr &A, const F *x, F *y, int nv, bool axpy, cudaStream_t s) {
     XG_DISPATCH(A, nv, {
         if (axpy)
-            launch<F, F, I, NV, 0, true>(A, x, k::EAxpy<F, NV>{{}, y}, s);
+            launch<F, F, I, NV, 0, true>(A, x, k::EAxpy<F, NV>(y), s);
         else
-            launch<F, F, I, NV, 0, true>(A, x, k::EStore<F, NV>{{}, y}, s);
+            launch<F, F, I, NV, 0, true>(A, x, k::EStore<F, NV>(y), s);
     });
 }
 template void spmv<double>(const DCsr &, const double *, double *, int, bool, cudaStream_t);

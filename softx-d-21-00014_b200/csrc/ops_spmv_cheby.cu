@@ -8,7 +8,7 @@ template <typename F>
 void cheby_first(const DCsr &A, const F *x, bool x_zero, const F *b, const F *isd, F c, F *rs,
                  F *t1s, int nv, cudaStream_t s) {
     XG_DISPATCH(A, nv, {
-        k::ECheby0<F, NV> e{{}, rs, t1s, b, isd, c};
+        k::ECheby0<F, NV> e(rs, t1s, b, isd, c);
         if (x_zero)
             launch_rows<F, NV, 0>(A.nrows, e, s);
         else
@@ -25,7 +25,7 @@ void cheby_step(const DCsr &A, const F *t1s, const F *rs, const F *isd, F c, F *
                 bool x_zero, int nv, cudaStream_t s) {
     XG_DISPATCH(A, nv, {
         launch<F, F, I, NV, 0>(
-            A, t1s, k::ECheby1<F, NV>{{}, out, rs, isd, c, (int)last, (int)x_zero}, s);
+            A, t1s, k::ECheby1<F, NV>(out, rs, isd, c, (int)last, (int)x_zero), s);
     });
 }
 template void cheby_step<double>(const DCsr &, const double *, const double *, const double *,

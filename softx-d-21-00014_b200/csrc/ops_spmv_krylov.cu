@@ -8,7 +8,7 @@ namespace ops {
 void group1(const DCsr &A, const double *x, const double *b, double *r0, double *p, double *r,
             double *sc, int nv, cudaStream_t s) {
     XG_DISPATCH(A, nv, {
-        launch<double, double, I, NV, 1>(A, x, k::EGroup1<NV>{r0, p, r, b, sc}, s);
+        launch<double, double, I, NV, 1>(A, x, k::EGroup1<NV>(r0, p, r, b, sc), s);
     });
 }
 
@@ -45,24 +45,24 @@ void group1_zero(uint64_t n, const double *b, double *r0, double *p, double *r, 
 void spmv_dot_alpha(const DCsr &A, const double *pa, double *v, const double *r0, double *sc,
                     int nv, cudaStream_t s) {
     XG_DISPATCH(A, nv, {
-        launch<double, double, I, NV, 1, true>(A, pa, k::EDotAlpha<NV>{v, r0, sc}, s);
+        launch<double, double, I, NV, 1, true>(A, pa, k::EDotAlpha<NV>(v, r0, sc), s);
     });
 }
 
 void spmv_dot_alpha(const DCsr &A, const float *pa, double *v, const double *r0, double *sc,
                     int nv, cudaStream_t s) {
     XG_DISPATCH(A, nv, {
-        launch<double, float, I, NV, 1>(A, pa, k::EDotAlpha<NV>{v, r0, sc}, s);
+        launch<double, float, I, NV, 1>(A, pa, k::EDotAlpha<NV>(v, r0, sc), s);
     });
 }
 
 void spmv_dot3(const DCsr &A, const float *sa, double *t, const double *s_, double *sc, int nv,
                cudaStream_t s) {
-    XG_DISPATCH(A, nv, { launch<double, float, I, NV, 3>(A, sa, k::EDot3<NV>{t, s_, sc}, s); });
+    XG_DISPATCH(A, nv, { launch<double, float, I, NV, 3>(A, sa, k::EDot3<NV>(t, s_, sc), s); });
 }
 
 void pcg_ap(const DCsr &A, const double *p, double *Ap, double *sc, int nv, cudaStream_t s) {
-    XG_DISPATCH(A, nv, { launch<double, double, I, NV, 1>(A, p, k::EPcgAp<NV>{Ap, p, sc}, s); });
+    XG_DISPATCH(A, nv, { launch<double, double, I, NV, 1>(A, p, k::EPcgAp<NV>(Ap, p, sc), s); });
 }
 
 void pcg_dots(uint64_t n, const double *r, const double *z, double *sc, bool first, int nv,
@@ -83,7 +83,7 @@ void rb_group1(uint64_t n, double *r, const double *v, const double *t, const do
 
 void spmv_dot3(const DCsr &A, const double *sa, double *t, const double *s_, double *sc, int nv,
                cudaStream_t s) {
-    XG_DISPATCH(A, nv, { launch<double, double, I, NV, 3>(A, sa, k::EDot3<NV>{t, s_, sc}, s); });
+    XG_DISPATCH(A, nv, { launch<double, double, I, NV, 3>(A, sa, k::EDot3<NV>(t, s_, sc), s); });
 }
 
 // --- canonical-order vector reductions ------------------------------------

@@ -8,7 +8,7 @@ template <typename F>
 void jacobi_sweep(const DCsr &A, const F *xin, F *xout, const F *b, const F *d, F relax, int nv,
                   cudaStream_t s) {
     XG_DISPATCH(A, nv, {
-        launch<F, F, I, NV, 0>(A, xin, k::EJacobi<F, NV>{{}, xout, xin, b, d, relax}, s);
+        launch<F, F, I, NV, 0>(A, xin, k::EJacobi<F, NV>(xout, xin, b, d, relax), s);
     });
 }
 template void jacobi_sweep<double>(const DCsr &, const double *, double *, const double *,
@@ -20,7 +20,7 @@ template void jacobi_sweep<float>(const DCsr &, const float *, float *, const fl
 void prolong_mixed(const DCsr &P, const float *xH, double *x, bool x_zero, int nv,
                    cudaStream_t s) {
     XG_DISPATCH(P, nv, {
-        launch<float, float, I, NV, 0>(P, xH, k::EProlongMixed<NV>{{}, x, (int)x_zero}, s);
+        launch<float, float, I, NV, 0>(P, xH, k::EProlongMixed<NV>(x, (int)x_zero), s);
     });
 }
 

@@ -10,9 +10,9 @@ void residual(const DCsr &A, const F *x, const F *b, F *r, int nv, double *norm_
               cudaStream_t s) {
     XG_DISPATCH(A, nv, {
         if (norm_out)
-            launch<F, F, I, NV, 1>(A, x, k::EResid<F, NV, true>{r, b, norm_out}, s);
+            launch<F, F, I, NV, 1>(A, x, k::EResid<F, NV, true>(r, b, norm_out), s);
         else
-            launch<F, F, I, NV, 0>(A, x, k::EResid<F, NV, false>{r, b, nullptr}, s);
+            launch<F, F, I, NV, 0>(A, x, k::EResid<F, NV, false>(r, b, nullptr), s);
     });
 }
 template void residual<double>(const DCsr &, const double *, const double *, double *, int,

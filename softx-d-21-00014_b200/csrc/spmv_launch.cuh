@@ -260,19 +260,25 @@ static uint8_t autotune(const DCsr &A, const FX *x, cudaStream_t s) {
     constexpr int VD = k::spmv_vk<FX, NV>();
     constexpr int VA = spmv_vk_alt<FX, NV>();
     DevBuf y(A.nrows * (uint64_t)NV * sizeof(F));
-    k::EStore<F, NV> e{{}, y.as<F>()};
+    k::EStore<F, NV> e(y.as<F>());
     cudaEvent_t e0, e1;
     XG_CUDA(cudaEventCreate(&e0));
     XG_CUDA(cudaEventCreate(&e1));
     float best = 1e30f;
     uint8_t code = 1;
     constexpr bool V8 = spmv_has_vk8<FX, NV, 0>() && VD != 8 && VA != 8;
-    // run index 3: the plane walk, where the matrix has one at this nv
-    const int nruns = walk_stride(A, (uint64_t)(k::CT / NV)) ? 4 : 3;
+    // run index 3: the plane walk, where the matrix has one at this nv. Fewer
+    // tiles than SMs times four leave each block at most one tile whatever the
+    // shape: runs of tiles would only take blocks away, and a second buffer is
+    // never filled, so those candidates are left out (their timings differed
+    // by noise alone).
+    const uint64_t tiles = (A.nrows + k::CT / NV - 1) / (uint64_t)(k::CT / NV);
+    const bool few = tiles <= 4ull * (uint64_t)ctx().sms;
+    const int nruns = few ? 1 : walk_stride(A, (uint64_t)(k::CT / NV)) ? 4 : 3;
     for (int alt = 0; alt < 3; ++alt)
         for (uint32_t nb = 1; nb <= 3; ++nb)
             for (int ri = 0; ri < nruns; ++ri) {
-                if ((alt == 1 && VA == VD) || (alt == 2 && !V8)) continue;
+                if ((alt == 1 && VA == VD) || (alt == 2 && !V8) || (few && nb == 2)) continue;
                 const uint32_t run = ri == 3 ? RUN_WALK : TUNE_RUNS[ri];
                 auto go = [&] {
                     if (alt == 2) {
@@ -325,22 +331,20 @@ static uint8_t autotune(const DCsr &A, const FX *x, cudaStream_t s) {
     return code;
 }
 
-// Vector loads of x need x aligned to VK elements; library vectors always are
-// (cudaMalloc). The entry points that take a caller's x (CALLER_X) fall back
-// to one right-hand side per thread for an x that is not (same results, same
-// reduction order).
-// FP64 x on short rows (fewer than 16 entries on average: 7-point stencils
-// and the like) takes four right-hand sides per thread: the staging buffers
-// are small enough for sixteen 64-thread blocks an SM, and the wider gathers
-// win; longer rows keep two.
+// Vector loads need x aligned to VK elements and the epilogue's vectors to 16
+// bytes; library vectors always are (cudaMalloc). The entry points that take a
+// caller's vectors (CALLER_X) fall back to one right-hand side per thread where
+// they are not (same results, same reduction order).
 template <typename F, typename FX, typename I, int NV, int NRED, bool CALLER_X, typename V,
           class Epi>
 static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s) {
-    // With dot products the grid is the canonical 1,184 blocks (one wave at
-    // eight an SM), so the threads a block has are the warps an SM keeps in
-    // flight: such kernels carry at most two right-hand sides a thread (FP32 x
-    // at four a thread measured 35 % slower on the 27-point 128^3 matrix).
-    constexpr int VK = NRED > 0 ? std::min(k::spmv_vk<FX, NV>(), 2) : k::spmv_vk<FX, NV>();
+    // Dot products: four right-hand sides a thread (kernels.cuh, register
+    // budget); two where a caller's x allows 16-byte gathers only.
+    constexpr int VK = NRED > 0 ? std::min(NV, 4) : k::spmv_vk<FX, NV>();
+    // The widest gathers, 32 bytes, where nothing was measured for the matrix.
+    constexpr int VW = std::min(NV, 32 / (int)sizeof(FX));
+    // the epilogue's vectors are read and written 16 bytes at a time too
+    const bool aligned = epi.aligned();
     if constexpr (NRED == 0) {
         if (A.wide_force && A.nrows * (uint64_t)NV <= WIDE_MAX_VALUES) {
             launch_wide<F, FX, I, NV, V>(A, x, epi, s);
@@ -352,13 +356,13 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
                 return;
             }
         if (A.walk_force && walk_stride(A, (uint64_t)(k::CT / NV)) &&
-            (VK == 1 || (uintptr_t)x % (VK * sizeof(FX)) == 0)) {
+            (VK == 1 || (aligned && (uintptr_t)x % (VK * sizeof(FX)) == 0))) {
             launch_vk<F, FX, I, NV, VK, NRED, V>(A, x, epi, s, 0, RUN_WALK);
             return;
         }
     }
     if constexpr (NRED == 0 && NV > 1) {
-        if (A.tune_on && (uintptr_t)x % (4 * sizeof(FX)) == 0) {
+        if (A.tune_on && aligned && (uintptr_t)x % 32 == 0) {
             int l = 0;
             while ((1 << l) < NV) ++l;
             uint8_t &t = A.tuned[sizeof(F) == 4][sizeof(FX) == 4][l];
@@ -385,11 +389,22 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
             }
         }
     }
-    constexpr uintptr_t ALIGN = VK * sizeof(FX);
-    constexpr bool SHORT4 = sizeof(FX) == 8 && VK == 2 && NV >= 4 && NRED == 0;
-    if (SHORT4 && A.nnz < 16 * A.nrows && (uintptr_t)x % (4 * sizeof(FX)) == 0) {
-        if constexpr (SHORT4) launch_vk<F, FX, I, NV, 4, NRED, V>(A, x, epi, s);
-    } else if (VK == 1 || (uintptr_t)x % ALIGN == 0) {
+    auto fits = [&](int vk) {
+        return vk == 1 || (aligned && (uintptr_t)x % (vk * sizeof(FX)) == 0);
+    };
+    if constexpr (NRED == 0 && VW != VK) {
+        if (fits(VW)) {
+            launch_vk<F, FX, I, NV, VW, NRED, V>(A, x, epi, s);
+            return;
+        }
+    }
+    if constexpr (NRED > 0 && CALLER_X && VK * sizeof(FX) > 16) {
+        if (!fits(VK) && fits(VK / 2)) {
+            launch_vk<F, FX, I, NV, VK / 2, NRED, V>(A, x, epi, s);
+            return;
+        }
+    }
+    if (fits(VK)) {
         launch_vk<F, FX, I, NV, VK, NRED, V>(A, x, epi, s);
     } else if constexpr (CALLER_X) {
         launch_vk<F, FX, I, NV, 1, NRED, V>(A, x, epi, s);
@@ -470,7 +485,7 @@ static uint8_t tune_stencil(const DCsr &A, const F *x, cudaStream_t s) {
     XG_CUDA(cudaStreamIsCapturing(s, &cs));
     if (cs != cudaStreamCaptureStatusNone) return 0;
     DevBuf y(A.nrows * (uint64_t)NV * sizeof(F));
-    k::EStore<F, NV> e{{}, y.as<F>()};
+    k::EStore<F, NV> e(y.as<F>());
     cudaEvent_t e0, e1;
     XG_CUDA(cudaEventCreate(&e0));
     XG_CUDA(cudaEventCreate(&e1));

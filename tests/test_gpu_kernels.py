@@ -62,6 +62,30 @@ def test_spmv_bit_exact(gpu, oracle, nv, col_bytes, ncols, f32):
         assert got.tobytes() == want.tobytes(), f"mode {mode}: {np.abs(got - want).max()}"
 
 
+@pytest.mark.parametrize("nv,f32", [(2, False), (4, True), (8, False), (8, True)])
+@pytest.mark.parametrize("dx,dy", [(1, 0), (0, 1), (2, 1)])
+def test_spmv_unaligned_vectors(gpu, oracle, nv, f32, dx, dy):
+    """A caller's x or y that starts dx or dy elements off a 16-byte boundary."""
+    import torch
+    rng = np.random.default_rng(nv + dx)
+    n = 700
+    row, col, val = random_csr(n, n, rng)
+    dt = np.float32 if f32 else np.float64
+    x, y0 = rng.standard_normal(n * nv).astype(dt), rng.standard_normal(n * nv).astype(dt)
+    A, keep = dev_csr(gpu, row, col, val, n, 2, f32)
+    xd = torch_dev(np.concatenate([np.zeros(dx, dt), x]))
+    for mode in (0, 1):
+        yd = torch_dev(np.concatenate([np.full(dy, 9.0, dt), y0]))
+        es = x.itemsize
+        gpu.call("XAMG_b200_spmv", C.byref(A), xd.data_ptr() + dx * es, yd.data_ptr() + dy * es,
+                 nv, mode, None)
+        torch.cuda.synchronize()
+        want = oracle.csr_ax_y(row, col, val.astype(dt), x, nv,
+                               axpy_y=(y0 if mode == 1 else None))
+        got = yd.cpu().numpy()
+        assert got[dy:].tobytes() == want.tobytes() and np.all(got[:dy] == 9.0)
+
+
 def test_spmv_edge_cases(gpu, oracle):
     import torch
     rng = np.random.default_rng(11)
