@@ -86,7 +86,8 @@ int XAMG_b200_dot(uint64_t n, int nv, const double *x, const double *y, double *
  * pool allocator, or a latency-bound loop where a cudaMalloc, which may
  * synchronise the device, is not allowed). No counterpart in the reference.
  * It allocates nothing: its scratch is a fixed __device__ array of this
- * library (1184 x 32 partial sums, 303,104 bytes, plus a counter) whose device
+ * library (1184 x 32 partial sums, 303,104 bytes, 32 x 32 sums of them, 8,192
+ * bytes, and counters) whose device
  * address is looked up on the first call on each device, so that first call
  * should precede any stream capture. x, y and dot_out (nv doubles) are device
  * arrays; nv must be 1, 2, 4, 8, 16 or 32 (XAMG_ERR_INVALID_ARG otherwise).

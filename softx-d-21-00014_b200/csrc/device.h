@@ -72,9 +72,10 @@ struct Lane {
 // lane (use_lane swaps them).
 struct Ctx {
     cudaStream_t stream = nullptr;
-    DevBuf red_part;    // canonical-reduction partials: BMAX x 32 x 3 doubles
-    DevBuf red_ticket;  // [0] reduction counter (zero between launches),
-                        // [1] tile-size scratch, [2] wait-timeout flag
+    DevBuf red_part;    // canonical-reduction partials: BMAX x 32 x 4 doubles, then
+                        // the groups' sums: 32 x 32 x 4
+    DevBuf red_ticket;  // [0] and [32..63] reduction counters (zero between
+                        // launches), [1] tile-size scratch, [2] wait-timeout flag
     DevBuf red_out;     // 96 doubles for reductions returned to the host
     double *pinned = nullptr;  // 256 doubles of pinned host memory
     int device = 0;
@@ -89,7 +90,8 @@ struct Ctx {
     // Makes lane i current (creating it on first use); lane 0 is the default.
     void use_lane(int i);
     k::RedArgs red() const {
-        return k::RedArgs{red_part.p, red_ticket.as<unsigned>(), red_ticket.as<unsigned>() + 2};
+        return k::RedArgs{red_part.p, red_ticket.as<unsigned>(), red_ticket.as<unsigned>() + 2,
+                          red_part.as<double>() + (size_t)k::BMAX * 32 * 4};
     }
     // Throws XAMG_ERR_TIMEOUT (and clears the flag) if a kernel's bounded wait
     // ran out since the last check; synchronises the stream.

@@ -21,8 +21,9 @@
 // dealt round-robin to B = min(ntiles, 1184) blocks (8 per SM on 148 SMs).
 // Dot products are accumulated per thread in tile order, combined within a
 // warp by an xor butterfly (offsets 16..NV), across the 8 warps in warp
-// order, and across blocks by the last block to finish: lane l sums blocks
-// l, l+32, ... and a full butterfly finishes. The order depends only on
+// order, and across blocks in 32 groups: group l sums blocks l, l+32, ... (its
+// last block to finish), and a full butterfly over the groups finishes (the
+// last group's). The order depends only on
 // (n, NV), so results are reproducible run to run and the CPU oracle can
 // replay it exactly.
 #pragma once
@@ -103,9 +104,13 @@ inline int canon_blocks(uint64_t n, int nv) {
 // ---------------------------------------------------------------------------
 struct RedArgs {
     void *part;              // [BMAX][32][4] partial sums (element type of the kernel)
-    unsigned *ticket;        // zero between launches
+    unsigned *ticket;        // [0] groups done, [RED_GROUP + l] blocks of group l done;
+                             // zero between launches
     unsigned *flag = nullptr;  // bit 0: a bounded wait ran out (read by the host)
+    void *groups = nullptr;    // [32][32][4] sums of the groups
 };
+constexpr int RED_GROUPS = 32, RED_GROUP = 32;
+constexpr int RED_TICKETS = RED_GROUP + RED_GROUPS;
 
 // A block may run the 256 canonical threads with CT/VK physical threads:
 // physical thread p plays canonical threads p*VK .. p*VK+VK-1 (right-hand
@@ -147,43 +152,55 @@ __device__ __forceinline__ void canon_partial(T (&acc)[VK][NRED], const RedArgs 
     __syncthreads();  // wsum is free for the next canonical block
 }
 
-// canon_final: after all of a launch's partials are written, the last
-// physical block to arrive sums the B partials (lane l sums l, l+32, ...,
-// then a full butterfly) and calls fin(k, sums of k).
+// canon_final: called by every thread after a canonical block's canon_partial.
+// The last block of each group (blocks l, l+32, ...) sums the group's partials,
+// one thread a sum, in block order; the last group to finish adds the groups by
+// a full butterfly and calls fin(k, sums of k). One block summing all B
+// partials by itself kept the launch waiting for NV*NRED*B loads from one SM:
+// the three dot products of 32 right-hand sides took 142 us with the SpMV's 70.
 template <typename T, int NV, int NRED, int NT, class Fin>
-__device__ __forceinline__ void canon_final(const RedArgs &ra, uint32_t B, const Fin &fin) {
-    constexpr int NW = NT / 32;
-    __shared__ T sums[NV * NRED];
+__device__ __forceinline__ void canon_final(const RedArgs &ra, uint32_t cb, uint32_t B,
+                                            const Fin &fin) {
+    constexpr int NW = NT / 32, NO = NV * NRED;
+    __shared__ T sums[NO];
     __shared__ int is_last;
     const T *part = (const T *)ra.part;
+    T *group = (T *)ra.groups;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t l = cb % RED_GROUPS, members = (B - l + RED_GROUPS - 1) / RED_GROUPS;
+    const uint32_t ngroups = B < (uint32_t)RED_GROUPS ? B : (uint32_t)RED_GROUPS;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = atomicAdd(&ra.ticket[RED_GROUP + l], 1u) == members - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int o = threadIdx.x; o < NO; o += NT) {
+        T a = T(0);
+#pragma unroll 8
+        for (uint32_t bb = l; bb < B; bb += RED_GROUPS)
+            a = add(a, ld_cg(&part[(size_t)bb * NO + o]));
+        group[l * NO + o] = a;
+    }
     __threadfence();
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned t = atomicAdd(ra.ticket, 1u);
-        is_last = (t == gridDim.x - 1);
+        ra.ticket[RED_GROUP + l] = 0u;
+        is_last = atomicAdd(&ra.ticket[0], 1u) == ngroups - 1;
     }
     __syncthreads();
     if (!is_last) return;
     __threadfence();
-    for (int o = warp; o < NV * NRED; o += NW) {
-        T a = T(0);
-        for (unsigned bb = lane; bb < B; bb += 32)
-            a = add(a, ld_cg(&part[(size_t)bb * NV * NRED + o]));
+#pragma unroll 4
+    for (int o = warp; o < NO; o += NW) {
+        T a = (uint32_t)lane < ngroups ? ld_cg(&group[lane * NO + o]) : T(0);
 #pragma unroll
         for (int off = 16; off >= 1; off >>= 1) a = add(a, shfl_xor(a, off));
         if (lane == 0) sums[o] = a;
     }
     __syncthreads();
-    if (threadIdx.x == 0) *ra.ticket = 0u;
+    if (threadIdx.x == 0) ra.ticket[0] = 0u;
     for (int kk = threadIdx.x; kk < NV; kk += NT) fin(kk, &sums[kk * NRED]);
-}
-
-// One canonical block per physical block (256 threads).
-template <typename T, int NV, int NRED, class Fin>
-__device__ __forceinline__ void canon_finish(T (&acc)[NRED], const RedArgs &ra, const Fin &fin) {
-    canon_partial<T, NV, NRED, 1>(reinterpret_cast<T(&)[1][NRED]>(acc), ra, blockIdx.x);
-    canon_final<T, NV, NRED, CT>(ra, gridDim.x, fin);
 }
 
 // ---------------------------------------------------------------------------
@@ -673,7 +690,10 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED>())
         __syncthreads();  // every reader is done with this tile's buffer
         if (nbuf == 1 && threadIdx.x == 0 && more) issue(nxt.j0, tile_end(nxt.r0));
         if constexpr (NRED > 0)
-            if (!more || an.left != at.left) canon_partial<F, NV, NRED, VK>(acc, ra, at.left);
+            if (!more || an.left != at.left) {
+                canon_partial<F, NV, NRED, VK>(acc, ra, at.left);
+                canon_final<F, NV, NRED, CT / VK>(ra, at.left, B, epi);
+            }
         at = an;
         an = ann;
         cur = nxt;
@@ -685,7 +705,6 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED>())
         if (threadIdx.x == 0)
             for (uint32_t u = n_used; u < n_issued; ++u) mbar_wait(&mbar[u % nbuf], (u / nbuf) & 1u);
     }
-    if constexpr (NRED > 0) canon_final<F, NV, NRED, CT / VK>(ra, B, epi);
 }
 
 // Warp-per-row SpMV for matrices with few rows (the coarse levels and their
@@ -801,20 +820,33 @@ static __global__ void k_tile_max(const uint32_t *__restrict__ row, uint64_t n, 
 // Element-wise canonical kernel (same schedule, no matrix). At most 64
 // registers a thread, so that four 256-thread blocks share an SM (the merged
 // group kernels with nv <= 8 take 76 registers left alone, three blocks);
-// these streaming kernels are bound by the loads in flight.
-template <typename F, int NV, int NRED, class Epi>
-__global__ void __launch_bounds__(CT, 4) k_rows(uint64_t n, Epi epi, RedArgs ra) {
-    constexpr int R = CT / NV;
-    const int rt = threadIdx.x / NV, k = threadIdx.x % NV;
+// these streaming kernels are bound by the loads in flight. With VK > 1 a
+// thread plays VK canonical threads of a row with 16-byte accesses (elemv): as
+// many threads an SM in blocks of CT/VK, VK times the bytes in flight.
+template <typename F, int NV, int NRED, class Epi, int VK = 1>
+__global__ void __launch_bounds__(CT / VK, 4 * VK) k_rows(uint64_t n, Epi epi, RedArgs ra) {
+    constexpr int R = CT / NV, G = NV / VK;
+    constexpr int NR = NRED > 0 ? NRED : 1;
+    const int rt = threadIdx.x / G, k0 = (threadIdx.x % G) * VK;
     const uint64_t ntiles = (n + R - 1) / R;
-    F acc[NRED > 0 ? NRED : 1];
+    F acc[VK][NR];
 #pragma unroll
-    for (int r = 0; r < (NRED > 0 ? NRED : 1); ++r) acc[r] = F(0);
+    for (int v = 0; v < VK; ++v)
+#pragma unroll
+        for (int r = 0; r < NR; ++r) acc[v][r] = F(0);
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint64_t i = tile * R + rt;
-        if (i < n) epi.elem(i, k, acc);
+        if (i < n) {
+            if constexpr (VK == 1)
+                epi.elem(i, k0, acc[0]);
+            else
+                epi.template elemv<VK>(i, k0, acc);
+        }
     }
-    if constexpr (NRED > 0) canon_finish<F, NV, NRED>(acc, ra, epi);
+    if constexpr (NRED > 0) {
+        canon_partial<F, NV, NRED, VK>(acc, ra, blockIdx.x);
+        canon_final<F, NV, NRED, CT / VK>(ra, blockIdx.x, gridDim.x, epi);
+    }
 }
 
 // Scalar-only kernel: one thread per right-hand side.
@@ -1125,6 +1157,55 @@ struct ECheby0 : EpiBase<ECheby0<F, NV>, F>, NoFin {
         rs[e] = rr;
         t1s[e] = mul(mul(c, rr), d);
     }
+    template <int VK, int NR>
+    __device__ void elemv(uint64_t i, int k0, F (&)[VK][NR]) const {
+        const uint64_t e = i * NV + k0;
+        const F d = isd[i];
+        const Vec<F, VK> bv = ldv<VK>(b + e);
+        Vec<F, VK> rr, t1;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            rr.v[v] = mul(mul(F(1), bv.v[v]), d);
+            t1.v[v] = mul(mul(c, rr.v[v]), d);
+        }
+        stv<VK>(rs + e, rr);
+        stv<VK>(t1s + e, t1);
+    }
+};
+
+// The same step from x = 0 with b still in double (the input of an FP32
+// multigrid preconditioner): b is rounded to float, kept in b32 for the rest
+// of the cycle, and the step is taken from the rounded value, in one pass
+// instead of a conversion and the step.
+template <int NV>
+struct ECheby0From64 : NoFin {
+    float *b32, *rs, *t1s;
+    const double *b;
+    const float *isd;
+    float c;
+    ECheby0From64(float *b32_, float *rs_, float *t1s_, const double *b_, const float *isd_,
+                  float c_)
+        : b32(b32_), rs(rs_), t1s(t1s_), b(b_), isd(isd_), c(c_) {}
+    template <int VK, int NR>
+    __device__ void elemv(uint64_t i, int k0, float (&)[VK][NR]) const {
+        const uint64_t e = i * NV + k0;
+        const float d = isd[i];
+        const Vec<double, VK> bv = ldv<VK>(b + e);
+        Vec<float, VK> bf, rr, t1;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            bf.v[v] = (float)bv.v[v];
+            rr.v[v] = mul(mul(1.0f, bf.v[v]), d);
+            t1.v[v] = mul(mul(c, rr.v[v]), d);
+        }
+        stv<VK>(b32 + e, bf);
+        stv<VK>(rs + e, rr);
+        stv<VK>(t1s + e, t1);
+    }
+    template <int NR>
+    __device__ void elem(uint64_t i, int k, float (&acc)[NR]) const {
+        elemv<1>(i, k, reinterpret_cast<float(&)[1][NR]>(acc));
+    }
 };
 
 // Chebyshev inner step i (chebyshev.inl:189-199):
@@ -1267,6 +1348,34 @@ struct EGroup4 {
         const double rv = sub(s[e], mul(om, t[e]));
         r[e] = rv;
         acc[0] = add(acc[0], mul(rv, r0[e]));
+    }
+    template <int VK, int NR>
+    __device__ void elemv(uint64_t i, int k0, double (&acc)[VK][NR]) const {
+        const uint64_t e = i * NV + k0;
+        const Vec<double, VK> sv = ldv<VK>(s + e), tv = ldv<VK>(t + e), r0v = ldv<VK>(r0 + e);
+        if constexpr (XUPD) {
+            Vec<double, VK> xv = ldv<VK>(x + e);
+            const Vec<PT, VK> pv = ldv<VK>(pa + e), qv = ldv<VK>(sa + e);
+#pragma unroll
+            for (int v = 0; v < VK; ++v) {
+                const double ac = sc[SC_ALPHA_C * SC_STRIDE + k0 + v];
+                const double oc = sc[SC_OMEGA_C * SC_STRIDE + k0 + v];
+                xv.v[v] = add(add(mul(ac, (double)pv.v[v]), mul(oc, (double)qv.v[v])),
+                              mul(1.0, xv.v[v]));
+            }
+            stv<VK>(x + e, xv);
+        }
+        Vec<double, VK> rv;
+#pragma unroll
+        for (int v = 0; v < VK; ++v) {
+            rv.v[v] = sub(sv.v[v], mul(sc[SC_OMEGA * SC_STRIDE + k0 + v], tv.v[v]));
+            acc[v][0] = add(acc[v][0], mul(rv.v[v], r0v.v[v]));
+        }
+        stv<VK>(r + e, rv);
+    }
+    bool aligned() const {
+        return aligned16(s) && aligned16(t) && aligned16(r0) && aligned16(r) &&
+               (!XUPD || (aligned16(x) && aligned16(pa) && aligned16(sa)));
     }
     __device__ void operator()(int k, const double *s1) const {
         double *S = sc;
@@ -1713,7 +1822,7 @@ __device__ __forceinline__ bool grid_sync(const GridSync &g, unsigned expected) 
 }
 
 // The last step of the canonical reduction run by every block for itself
-// (the same sums, in the same order, as canon_final's last block), with the
+// (the same sums, in the same order, as canon_final's), with the
 // finaliser writing the block's own copy of the scalar block: no block
 // depends on another's finaliser.
 template <int NV, int NRED, class Fin>

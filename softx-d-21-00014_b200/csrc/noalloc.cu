@@ -22,9 +22,10 @@
 // Inputs and the output are the caller's device arrays.
 //
 // Limits: nv must be 1, 2, 4, 8, 16 or 32; the array holds 1184 x 32 partial
-// sums (303,104 bytes) plus the counter, enough for every row count since the
-// reduction uses at most 1184 blocks. Every call uses the same array, and the
-// counter is cleared at the start of each call: two calls whose kernels overlap
+// sums (303,104 bytes), 32 x 32 group sums (8,192 bytes) and the counters, enough
+// for every row count since the reduction uses at most 1184 blocks. Every call
+// uses the same array, and the counters are cleared at the start of each call:
+// two calls whose kernels overlap
 // on the GPU (for example on two streams) race and give wrong results.
 #include <type_traits>
 
@@ -34,7 +35,9 @@ namespace xg {
 namespace {
 
 constexpr int NOALLOC_PARTIALS = k::BMAX * 32;         // doubles of partial sums
-constexpr int NOALLOC_WORDS = NOALLOC_PARTIALS + 32;   // + counter area
+constexpr int NOALLOC_GROUPS = k::RED_GROUPS * 32;     // and of group sums
+constexpr int NOALLOC_WORDS = NOALLOC_PARTIALS + NOALLOC_GROUPS + 32;  // + counters
+static_assert(k::RED_TICKETS * sizeof(unsigned) <= 32 * sizeof(double), "counter area");
 
 static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_WORDS];
 
@@ -64,11 +67,14 @@ cudaError_t load_dot_kernel() {
 template <int NV>
 int launch_dot(uint64_t n, const double *x, const double *y, double *out, double *scratch,
                cudaStream_t s) {
-    unsigned *ticket = (unsigned *)(scratch + NOALLOC_PARTIALS);
-    if (cudaMemsetAsync(ticket, 0, sizeof(unsigned), s) != cudaSuccess) return XAMG_ERR_CUDA;
+    double *groups = scratch + NOALLOC_PARTIALS;
+    unsigned *ticket = (unsigned *)(groups + NOALLOC_GROUPS);
+    if (cudaMemsetAsync(ticket, 0, k::RED_TICKETS * sizeof(unsigned), s) != cudaSuccess)
+        return XAMG_ERR_CUDA;
     const int B = k::canon_blocks(n, NV);
     k::k_rows<double, NV, 1, k::EDot<double, NV>>
-        <<<B, k::CT, 0, s>>>(n, k::EDot<double, NV>{x, y, out}, k::RedArgs{scratch, ticket});
+        <<<B, k::CT, 0, s>>>(n, k::EDot<double, NV>{x, y, out},
+                             k::RedArgs{scratch, ticket, nullptr, groups});
     return cudaGetLastError() == cudaSuccess ? XAMG_OK : XAMG_ERR_CUDA;
 }
 

@@ -115,6 +115,9 @@ void jacobi_zero(uint64_t n, F *x, const F *b, const F *d, F relax, int nv, cuda
 template <typename F>
 void cheby_first(const DCsr &A, const F *x, bool x_zero, const F *b, const F *isd, F c, F *rs,
                  F *t1s, int nv, cudaStream_t s);
+// the first step from x = 0 with b in double: also leaves float(b) in b32
+void cheby_first_from64(uint64_t n, const double *b, float *b32, const float *isd, float c,
+                        float *rs, float *t1s, int nv, cudaStream_t s);
 template <typename F>
 void cheby_step(const DCsr &A, const F *t1s, const F *rs, const F *isd, F c, F *out, bool last,
                 bool x_zero, int nv, cudaStream_t s);

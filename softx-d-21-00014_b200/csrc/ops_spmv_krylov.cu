@@ -109,7 +109,8 @@ void group4(uint64_t n, const double *s_, const double *t, const double *r0, dou
             double *x, const float *pa, const float *sa, double *sc, int nv, cudaStream_t s) {
     dispatch_nv(nv, [&](auto nvc) {
         constexpr int NV = decltype(nvc)::value;
-        launch_rows<double, NV, 1>(n, k::EGroup4<NV, true, float>{s_, t, r0, r, x, pa, sa, sc}, s);
+        launch_rows<double, NV, 1, (NV > 1 ? 2 : 1)>(
+            n, k::EGroup4<NV, true, float>{s_, t, r0, r, x, pa, sa, sc}, s);
     });
 }
 
@@ -118,10 +119,18 @@ void group4(uint64_t n, const double *s_, const double *t, const double *r0, dou
             cudaStream_t s) {
     dispatch_nv(nv, [&](auto nvc) {
         constexpr int NV = decltype(nvc)::value;
-        if (with_x)
-            launch_rows<double, NV, 1>(n, k::EGroup4<NV, true>{s_, t, r0, r, x, pa, sa, sc}, s);
+        constexpr int VK = NV > 1 ? 2 : 1;
+        const k::EGroup4<NV, true> ex{s_, t, r0, r, x, pa, sa, sc};
+        const k::EGroup4<NV, false> e{s_, t, r0, r, x, pa, sa, sc};
+        // a caller's vectors (the kernel-level entry point) may be unaligned
+        if (with_x && ex.aligned())
+            launch_rows<double, NV, 1, VK>(n, ex, s);
+        else if (with_x)
+            launch_rows<double, NV, 1>(n, ex, s);
+        else if (e.aligned())
+            launch_rows<double, NV, 1, VK>(n, e, s);
         else
-            launch_rows<double, NV, 1>(n, k::EGroup4<NV, false>{s_, t, r0, r, x, pa, sa, sc}, s);
+            launch_rows<double, NV, 1>(n, e, s);
     });
 }
 

@@ -37,8 +37,8 @@ void DVec::alloc(uint64_t n_, int nv_, bool f32_) {
 static void lane_create(cudaStream_t &stream, DevBuf &part, DevBuf &ticket, DevBuf &out,
                         double *&pinned) {
     XG_CUDA(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
-    part.alloc((size_t)k::BMAX * 32 * 4 * sizeof(double));
-    ticket.alloc(sizeof(unsigned) * 4);
+    part.alloc((size_t)(k::BMAX + k::RED_GROUPS) * 32 * 4 * sizeof(double));
+    ticket.alloc(sizeof(unsigned) * k::RED_TICKETS);
     out.alloc(128 * sizeof(double));
     XG_CUDA(cudaMemsetAsync(ticket.p, 0, ticket.bytes, stream));
     XG_CUDA(cudaMallocHost((void **)&pinned, 256 * sizeof(double)));

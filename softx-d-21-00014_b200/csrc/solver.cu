@@ -314,6 +314,9 @@ struct Chebyshev : public SolverBase {
     DevBuf isd;
     double min_eig = 0, max_eig = 0;
     std::vector<F> coef;
+    // set by the multigrid for its next call: the input b is still in double
+    // here and is rounded into b by the first step (x zero-flagged)
+    const double *from64 = nullptr;
     void setup_from(const HCsr &hA) {
         if (f32)
             upload(isd, inv_diag_f32(hA, true), S());
@@ -339,8 +342,16 @@ struct Chebyshev : public SolverBase {
         }
         DVec &rs = buf[0];
         DVec *t1s = &buf[1], *other = &buf[2];
-        ops::cheby_first<F>(*A, x.p<F>(), x_zero, b.p<F>(), isd.as<F>(), coef[order - 1],
-                            rs.p<F>(), t1s->p<F>(), NV, S());
+        const double *b64 = from64;
+        from64 = nullptr;
+        if constexpr (std::is_same<F, float>::value) {
+            if (b64)
+                ops::cheby_first_from64(n, b64, b.p<float>(), isd.as<float>(), coef[order - 1],
+                                        rs.p<float>(), t1s->p<float>(), NV, S());
+        }
+        if (!b64)
+            ops::cheby_first<F>(*A, x.p<F>(), x_zero, b.p<F>(), isd.as<F>(), coef[order - 1],
+                                rs.p<F>(), t1s->p<F>(), NV, S());
         if (order == 1) {
             ops::add_into<F>(x.p<F>(), t1s->p<F>(), x.elems(), x_zero, S());
         } else {
@@ -664,15 +675,27 @@ void MultiGrid::cycle(int level, DVec &x, DVec &b, int cyc, const std::vector<do
     post[level]->solve(x, b, iconv);
 }
 
+// Rounds the preconditioner's double input b into b32, or leaves that to the
+// first step of the finest level's Chebyshev pre-smoother where the cycle
+// starts with it from x = 0.
+void MultiGrid::take_input(DVec &b, bool x_zero) {
+    b32.zero = b.zero;
+    b32.init = true;
+    if (b.zero) return;
+    auto *ch = dynamic_cast<Chebyshev<float> *>(pre[0].get());
+    if (ch && x_zero && cfg.mg_cycle != 1 && !(ch->cfg.convergence_check && ch->cfg.convergence_info))
+        ch->from64 = b.p<double>();
+    else
+        ops::convert<float, double>(b32.p<float>(), b.p<double>(), b.elems(), S());
+}
+
 // The gpu_precond_f32 = 1 preconditioner with its result left in float in
 // x32 (a caller's buffer): the same cycles as solve(); a caller that reads
 // x32 widened exactly sees the values solve() would write into x.
 void MultiGrid::solve_to32(DVec &x32o, DVec &b, const std::vector<double> &conv) {
     reset_stats();
     std::vector<double> iconv = conv;
-    b32.zero = b.zero;
-    if (!b.zero) ops::convert<float, double>(b32.p<float>(), b.p<double>(), b.elems(), S());
-    b32.init = true;
+    take_input(b, x32o.zero);
     x32o.init = true;
     do {
         ++st.iters;
@@ -688,11 +711,10 @@ void MultiGrid::solve(DVec &x, DVec &b, const std::vector<double> &conv) {
     if (full32) {
         // preconditioner in float throughout: convert the input, cycle, convert
         // the result back (zero flags carried across)
-        b32.zero = b.zero;
-        if (!b.zero) ops::convert<float, double>(b32.p<float>(), b.p<double>(), b.elems(), S());
+        take_input(b, x.zero);
         x32.zero = x.zero;
         if (!x.zero) ops::convert<float, double>(x32.p<float>(), x.p<double>(), x.elems(), S());
-        b32.init = x32.init = true;
+        x32.init = true;
         do {
             ++st.iters;
             cycle(0, x32, b32, cfg.mg_cycle, iconv);

@@ -80,6 +80,7 @@ class MultiGrid : public SolverBase {
 
   private:
     void cycle(int level, DVec &x, DVec &b, int cyc, const std::vector<double> &iconv);
+    void take_input(DVec &b, bool x_zero);
 };
 
 // A preconditioner application captured as a CUDA graph: the kernels that

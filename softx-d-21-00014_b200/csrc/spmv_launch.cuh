@@ -577,11 +577,13 @@ static void launch(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s) {
     launch_v<F, FX, I, NV, NRED, CALLER_X, F>(A, x, epi, s);
 }
 
-template <typename F, int NV, int NRED, class Epi>
+// VK: right-hand sides a thread carries (16-byte accesses; the epilogue's
+// vectors aligned to that).
+template <typename F, int NV, int NRED, int VK = 1, class Epi>
 static void launch_rows(uint64_t n, const Epi &epi, cudaStream_t s) {
     if (n == 0) return;
     const int B = k::canon_blocks(n, NV);
-    k::k_rows<F, NV, NRED, Epi><<<B, k::CT, 0, s>>>(n, epi, ctx().red());
+    k::k_rows<F, NV, NRED, Epi, VK><<<B, k::CT / VK, 0, s>>>(n, epi, ctx().red());
     XG_CUDA(cudaGetLastError());
     ++g_kernel_launches;
 }
