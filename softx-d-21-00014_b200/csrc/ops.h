@@ -128,16 +128,31 @@ void prolong_mixed(const DCsr &P, const float *xH, double *x, bool x_zero, int n
 
 // HSGS: forward+backward sweeps over the Gauss-Seidel blocks. t is b -
 // A_offblock x_old; xin is x itself, or null for a sweep from x = 0 (t is then
-// b). plan: the blocks' sizes.
+// b). plan: the blocks' sizes. Adiag's rows are padded to multiples of four
+// entries (value 0, the column one past the block's rows) where hsgs_can_pad says
+// that blocks of those sizes fit in shared memory; otherwise its rows are as they
+// are and the sweep runs from global memory.
 struct HsgsPlan {
     uint64_t n = 0;
     uint32_t rows = 0;        // rows of a block (the last one may be shorter)
-    uint32_t ent_max[6] = {}; // most in-block entries of 2^l consecutive blocks
+    uint32_t ent_max[6] = {}; // most padded in-block entries of 2^l consecutive blocks
+    bool padded = false;
 };
+template <typename F>
+bool hsgs_can_pad(const HsgsPlan &plan, int nv);
 template <typename F>
 void hsgs_sweep(const DCsr &Adiag, const HsgsPlan &plan, const uint64_t *boff, int nblocks,
                 const F *t, const F *xin, F *x, const F *d, const double *relax_sc, int nv,
                 cudaStream_t s);
+
+// The same sweep with its lagged term b - A_offblock xin formed inside, into
+// another vector than xin; hsgs_can_fuse: whether the blocks allow it.
+template <typename F>
+bool hsgs_can_fuse(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, int nv);
+template <typename F>
+void hsgs_fused_sweep(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, const F *b,
+                      const F *xin, F *xout, const F *d, const double *relax_sc, int nv,
+                      cudaStream_t s);
 
 // Dense y = A_inv x (Direct coarse solve)
 template <typename F>

@@ -196,6 +196,7 @@ struct Hsgs : public SolverBase {
     std::vector<double> relax_on_dev;  // what relax_dev holds (host mirror)
     DCsr Adiag, Aoff;
     ops::HsgsPlan plan;
+    bool fuse = false;  // the lagged term inside the sweep's kernel
     int nblocks = 1;
     void setup_from(const HCsr &hA) {
         const uint64_t rows = cfg.gpu_hsgs_rows > 0 ? (uint64_t)cfg.gpu_hsgs_rows : 32;
@@ -240,18 +241,43 @@ struct Hsgs : public SolverBase {
             dg.row[i + 1] = (uint32_t)dg.col.size();
             od.row[i + 1] = (uint32_t)od.col.size();
         }
-        // blocks are cs rows each, the last one short (split_range_f64)
+        // blocks are cs rows each, the last one short (split_range_f64); their
+        // rows padded to whole chunks (hsgs.cuh)
         plan.n = n;
         plan.rows = (uint32_t)std::min<uint64_t>(cs, n);
+        auto padded = [&](uint64_t i) {
+            const uint32_t len = dg.row[i + 1] - dg.row[i];
+            return std::max<uint32_t>(4, (len + 3) / 4 * 4);
+        };
         for (int l = 0; l < 6; ++l) {
             const uint64_t per = (uint64_t)plan.rows << l;
             plan.ent_max[l] = 0;
-            for (uint64_t r = 0; r < n; r += per)
-                plan.ent_max[l] = std::max(plan.ent_max[l],
-                                           dg.row[std::min(n, r + per)] - dg.row[r]);
+            for (uint64_t r = 0; r < n; r += per) {
+                uint32_t e = 0;
+                for (uint64_t i = r; i < std::min(n, r + per); ++i) e += padded(i);
+                plan.ent_max[l] = std::max(plan.ent_max[l], e);
+            }
+        }
+        plan.padded = ops::hsgs_can_pad<F>(plan, NV);
+        if (plan.padded) {
+            HCsr p;
+            p.nrows = n;
+            p.ncols = plan.rows + 1;
+            p.row.assign(n + 1, 0);
+            for (uint64_t i = 0; i < n; ++i) p.row[i + 1] = p.row[i] + padded(i);
+            p.col.assign(p.row[n], plan.rows);
+            p.val.assign(p.row[n], 0.0);
+            for (uint64_t i = 0; i < n; ++i)
+                for (uint64_t j = dg.row[i]; j < dg.row[i + 1]; ++j) {
+                    p.col[p.row[i] + (j - dg.row[i])] = dg.col[j];
+                    p.val[p.row[i] + (j - dg.row[i])] = dg.val[j];
+                }
+            std::swap(dg, p);
         }
         upload_csr(dg, Adiag, f32, cfg.gpu_index_compress, S());
-        upload_csr(od, Aoff, f32, cfg.gpu_index_compress, S(), cfg.gpu_spmv_tune);
+        // absolute columns: a fused sweep reads off-block entries without their rows
+        upload_csr(od, Aoff, f32, std::min(cfg.gpu_index_compress, 1), S(), cfg.gpu_spmv_tune);
+        fuse = ops::hsgs_can_fuse<F>(Adiag, Aoff, plan, NV);
         upload(boff, off, S());
         if (f32)
             upload(d, inv_diag_f32(hA, false), S());
@@ -263,6 +289,48 @@ struct Hsgs : public SolverBase {
                                 cudaMemcpyHostToDevice, S()));
         alloc_buffers(2);
         XG_CUDA(cudaStreamSynchronize(S()));
+    }
+    // The sweeps without a convergence test: x alternates between x and
+    // buf[1], sweep j landing in x when (m - j) is even so that the last one
+    // does; the first sweep from x = 0 has no lagged term.
+    void solve_fused(DVec &x, DVec &b, const std::vector<double> &iconv, bool ones) {
+        std::vector<double> relax_h(NV, (double)(F)cfg.relax);
+        if (!ones)
+            for (int k = 0; k < NV; ++k) relax_h[k] = (double)(F)(relax_h[k] * iconv[k]);
+        set_relax(relax_h);
+        const int m = std::max(1, cfg.max_iters);
+        DVec &T = buf[1];
+        auto tgt = [&](int j) -> DVec & { return ((m - j) % 2 == 0) ? x : T; };
+        DVec *cur = &x;
+        int j = 1;
+        if (x.zero) {
+            DVec &o = tgt(1);
+            ops::hsgs_sweep<F>(Adiag, plan, boff.as<uint64_t>(), nblocks, b.p<F>(), nullptr,
+                               o.p<F>(), d.as<F>(), relax_dev.as<double>(), NV, S());
+            cur = &o;
+            j = 2;
+        } else if ((m - 1) % 2 == 0) {
+            ops::convert<F, F>(T.p<F>(), x.p<F>(), x.elems(), S());
+            cur = &T;
+        }
+        for (; j <= m; ++j) {
+            DVec &o = tgt(j);
+            ops::hsgs_fused_sweep<F>(Adiag, Aoff, plan, b.p<F>(), cur->p<F>(), o.p<F>(),
+                                     d.as<F>(), relax_dev.as<double>(), NV, S());
+            cur = &o;
+        }
+        st.iters = m;
+        x.zero = false;
+        x.init = true;
+    }
+    // The relaxation factors on the device, refreshed whenever they differ, so
+    // a solve that starts with every right-hand side active does not inherit
+    // the factors an earlier solve froze.
+    void set_relax(const std::vector<double> &relax_h) {
+        if (std::equal(relax_h.begin(), relax_h.end(), relax_on_dev.begin())) return;
+        std::copy(relax_h.begin(), relax_h.end(), relax_on_dev.begin());
+        XG_CUDA(cudaMemcpyAsync(relax_dev.p, relax_on_dev.data(), NV * sizeof(double),
+                                cudaMemcpyHostToDevice, S()));
     }
     void solve(DVec &x, DVec &b, const std::vector<double> &conv) override {
         reset_stats();
@@ -276,19 +344,16 @@ struct Hsgs : public SolverBase {
             residual_norm<F>(*A, x, b, r, NV, rho0.data());
             if (host_converged(*this, rho0.data(), rho0.data(), iconv)) return;
         }
+        if (fuse && !cfg.convergence_check) {
+            solve_fused(x, b, iconv, ones);
+            return;
+        }
         do {
             ++st.iters;
-            // scal(iconv, relax_conv) (hsgs.inl:102); the device copy is
-            // refreshed whenever it differs, so a solve that starts with every
-            // right-hand side active does not inherit the factors an earlier
-            // solve froze
+            // scal(iconv, relax_conv) (hsgs.inl:102)
             if (!ones || cfg.convergence_check)
                 for (int k = 0; k < NV; ++k) relax_h[k] = (double)(F)(relax_h[k] * iconv[k]);
-            if (!std::equal(relax_h.begin(), relax_h.end(), relax_on_dev.begin())) {
-                std::copy(relax_h.begin(), relax_h.end(), relax_on_dev.begin());
-                XG_CUDA(cudaMemcpyAsync(relax_dev.p, relax_on_dev.data(), NV * sizeof(double),
-                                        cudaMemcpyHostToDevice, S()));
-            }
+            set_relax(relax_h);
             // x zero-flagged: no lagged term, t = 1*b + (-1)*0 = b, and the
             // sweep starts from x = 0 (blas2.h:226-262)
             if (!x.zero)
