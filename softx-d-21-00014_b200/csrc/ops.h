@@ -17,9 +17,14 @@ void wait_selftest(uint64_t limit_ns, cudaStream_t s);
 // The persistent preconditioned BiCGStab (csrc/persist.cu): whether the
 // matrix's canonical blocks can all be resident at once, and the launch.
 // share: canonical blocks each physical block plays (gpu_persistent).
+// pbicgstab_exchange_bytes: size of the exchange buffer of the register-resident
+// form (0: the system does not take that form); the launch takes that form where
+// it is given one. The buffer's 8-byte tags must all be below tag0; a launch uses
+// fewer than 2^36 tags.
 bool pbicgstab_persist_fits(const DCsr &A, int nv, int share);
-void pbicgstab_persist(const DCsr &A, const k::PersistArgs &P, int nv, int share,
-                       cudaStream_t s);
+size_t pbicgstab_exchange_bytes(const DCsr &A, int nv, int sweeps, int share);
+void pbicgstab_persist(const DCsr &A, const k::PersistArgs &P, int nv, int share, void *exchange,
+                       uint64_t tag0, cudaStream_t s);
 // A grid barrier that one block never reaches: its waits run out after
 // limit_ns and raise *flag.
 void grid_selftest(unsigned *count_gen, unsigned *flag, uint64_t limit_ns, cudaStream_t s);

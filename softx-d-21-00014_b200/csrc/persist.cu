@@ -1,5 +1,7 @@
-// Launchers of the persistent preconditioned BiCGStab (k_pbicgstab_persist,
-// csrc/kernels.cuh) and of its grid barrier's self-test.
+// Launchers of the persistent preconditioned BiCGStab (k_pbicgstab_reg,
+// csrc/persist_reg.cuh, and k_pbicgstab_persist, csrc/kernels.cuh) and of its
+// grid barrier's self-test.
+#include "persist_reg.cuh"
 #include "spmv_launch.cuh"
 
 namespace xg {
@@ -26,17 +28,67 @@ bool pbicgstab_persist_fits(const DCsr &A, int nv, int share) {
     return ok;
 }
 
-void pbicgstab_persist(const DCsr &A, const k::PersistArgs &P, int nv, int share,
-                       cudaStream_t s) {
+// The register-resident form takes systems of at most one tile an SM (n * nv up
+// to 148 * 256) with a tile's entries in shared memory, and at most four Jacobi
+// sweeps; launches that share blocks (gpu_persistent > 1), larger systems and
+// more sweeps keep their vectors in global memory.
+constexpr uint32_t REG_SMEM_MAX = 200u * 1024u;
+
+template <int NV, typename I>
+static uint32_t reg_blocks(const DCsr &A, int sweeps, int share, uint32_t &smem, uint32_t &cap) {
+    constexpr uint64_t R = k::CT / NV;
+    const uint64_t ntiles = (A.nrows + R - 1) / R;
+    if (share > 1 || sweeps > k::REG_MAX_SWEEPS) return 0;
+    if (ntiles == 0 || ntiles > (uint64_t)ctx().sms) return 0;
+    if (std::max(A.ncols, A.nrows) * (uint64_t)NV >= (1ull << 32)) return 0;
+    cap = tile_max(A, NV, ctx().stream);
+    if ((uint64_t)cap * 12 > REG_SMEM_MAX) return 0;
+    smem = cap * 12;
+    auto kern = k::k_pbicgstab_reg<NV, I>;
+    static bool big_smem = false;  // one flag per instantiation
+    if (!big_smem) {
+        XG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     (int)REG_SMEM_MAX));
+        big_smem = true;
+    }
+    const int res = resident_blocks(kern, k::CT, smem);
+    return res >= 1 ? (uint32_t)ntiles : 0;
+}
+
+size_t pbicgstab_exchange_bytes(const DCsr &A, int nv, int sweeps, int share) {
+    size_t bytes = 0;
+    XG_DISPATCH(A, nv, {
+        uint32_t smem;
+        uint32_t cap;
+        const uint32_t blocks = reg_blocks<NV, I>(A, sweeps, share, smem, cap);
+        if (blocks) bytes = k::reg_exchange_values<NV>(A.nrows, blocks, sweeps) * sizeof(k::Tagged);
+    });
+    return bytes;
+}
+
+void pbicgstab_persist(const DCsr &A, const k::PersistArgs &P, int nv, int share, void *exchange,
+                       uint64_t tag0, cudaStream_t s) {
     XG_DISPATCH(A, nv, {
         const int B = k::canon_blocks(A.nrows, NV);
         k::CsrArgs<double> a = A.args<double>();
         k::PersistArgs p = P;
         p.B = (uint32_t)B;
-        void *args[] = {(void *)&a, (void *)&p};
-        XG_CUDA(cudaLaunchCooperativeKernel((const void *)k::k_pbicgstab_persist<NV, I>,
-                                            dim3((unsigned)grid_of(B, share)), dim3(k::CT), args,
-                                            0, s));
+        if (exchange) {
+            uint32_t smem = 0;
+            uint32_t cap = 0;
+            const uint32_t blocks = reg_blocks<NV, I>(A, P.sweeps, share, smem, cap);
+            XG_REQUIRE(blocks == (uint32_t)B, XAMG_ERR_INTERNAL, "register-resident BiCGStab");
+            k::Tagged *x = (k::Tagged *)exchange;
+            unsigned long long t0 = tag0;
+            void *args[] = {(void *)&a, (void *)&p, (void *)&x, (void *)&t0, (void *)&cap};
+            XG_CUDA(cudaLaunchCooperativeKernel((const void *)k::k_pbicgstab_reg<NV, I>,
+                                                dim3(blocks), dim3(k::CT), args, smem, s));
+        } else {
+            void *args[] = {(void *)&a, (void *)&p};
+            XG_CUDA(cudaLaunchCooperativeKernel((const void *)k::k_pbicgstab_persist<NV, I>,
+                                                dim3((unsigned)grid_of(B, share)), dim3(k::CT),
+                                                args, 0, s));
+        }
         ++g_kernel_launches;
     });
 }

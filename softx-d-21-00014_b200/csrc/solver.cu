@@ -1362,7 +1362,15 @@ void Krylov::run_persistent(DVec &x) {
     P.rel_tol = cfg.rel_tol;
     P.ra = ra;
     P.gs = k::GridSync{psync.as<unsigned long long>(), ra.flag, 1000000000ull};
-    ops::pbicgstab_persist(*A, P, NV, cfg.gpu_persistent, s);
+    // the register-resident form's exchange buffer: zeroed when allocated, its
+    // tags then grow from launch to launch
+    const size_t xb = ops::pbicgstab_exchange_bytes(*A, NV, P.sweeps, cfg.gpu_persistent);
+    if (xb > pexchange.bytes) {
+        pexchange.alloc(xb);
+        XG_CUDA(cudaMemsetAsync(pexchange.p, 0, xb, s));
+    }
+    ops::pbicgstab_persist(*A, P, NV, cfg.gpu_persistent, xb ? pexchange.p : nullptr,
+                           ++plaunches << 36, s);
     double out[97];
     XG_CUDA(cudaMemcpyAsync(out, pout.p, sizeof(out), cudaMemcpyDeviceToHost, s));
     ctx().check_flags();  // synchronises; XAMG_ERR_TIMEOUT if a grid wait ran out

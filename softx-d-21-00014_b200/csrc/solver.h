@@ -162,6 +162,8 @@ class Krylov : public SolverBase {
     bool persistent_ok() const;
     void run_persistent(DVec &x);
     DevBuf psync, pout;  // grid barrier counters; the launch's statistics
+    DevBuf pexchange;    // exchange buffer of the register-resident form
+    uint64_t plaunches = 0;  // its launches, the high bits of their tags
     MGraph &step_graph(const std::tuple<int, bool, const void *> &key);
     void run_graphed(MGraph &g, DVec *x, const std::function<void()> &body);
     // per (out, in, in.zero, lane): a graph's kernels carry its lane's scratch

@@ -60,6 +60,40 @@ def test_persistent_equals_stepwise(gpu, method, prec, nv, sweeps, grid, cap, sh
         assert true_rel_res(row, col, val, x1, b, nv).max() <= 1e-7
 
 
+@pytest.mark.parametrize("stencil,nv,grid,sweeps", [(27, 1, (32, 31, 33), None),
+                                                    (7, 16, (15, 14, 11), 1), (7, 32, (11, 10, 9), 2),
+                                                    (7, 8, (17, 16, 15), 4), (7, 8, (17, 16, 15), 5),
+                                                    (7, 4, (40, 39, 38), None)])
+def test_persistent_forms(gpu, stencil, nv, grid, sweeps):
+    """The register-resident form at its edges (nearly one block an SM, all lanes
+    of a warp on one row, long rows, as many Jacobi sweeps as it takes) and what
+    is beyond it (one sweep more, a larger system): the bits of the step-by-step
+    solve."""
+    row, col, val = gpu.generate_diffusion(stencil, *grid, 1.0, 1.0, 4)
+    n = len(row) - 1
+    b = np.random.default_rng(nv).uniform(-1, 1, n * nv)
+    x0, s0, _ = gpu_solve(gpu, row, col, val, nv,
+                          params("MergedPBiCGStab", True, 0, sweeps=sweeps), b)
+    x1, s1, _ = gpu_solve(gpu, row, col, val, nv,
+                          params("MergedPBiCGStab", True, 1, sweeps=sweeps), b)
+    assert s0["iters"] == s1["iters"] and s1["conv"].all()
+    assert s0["rel_res"].tobytes() == s1["rel_res"].tobytes()
+    assert x0.tobytes() == x1.tobytes()
+    # another right-hand side on the same solver: nothing is left of the first solve
+    M, X, B = matrix_and_vectors(gpu, row, col, val, nv)
+    S2 = gpu.Solver(M, gpu.Params(params("MergedPBiCGStab", True, 1, sweeps=sweeps)), X, B)
+    for rhs in (b[::-1].copy(), b):
+        B.upload(rhs)
+        X.set(0.0)
+        S2.solve()
+    assert X.download().tobytes() == x0.tobytes()
+
+
+def matrix_and_vectors(gpu, row, col, val, nv):
+    M = gpu.Matrix(row, col, val)
+    return M, gpu.Vector(M.n, nv, M.part), gpu.Vector(M.n, nv, M.part)
+
+
 def test_grid_barrier_wait_runs_out(gpu):
     t = C.c_int(-1)
     gpu.call("XAMG_b200_grid_selftest", 0.05, C.byref(t))
