@@ -20,6 +20,8 @@
 // order (a fixed order, no workspace) and applies the epilogue. Every wait is
 // bounded (global timer); a wait that runs out raises the library's timeout flag
 // and the CTA still frees its TMEM before it exits.
+#include <algorithm>
+
 #include <cuda.h>
 #include <cudaTypedefs.h>
 #include <cuda_bf16.h>
@@ -441,6 +443,52 @@ CUtensorMap make_map(const void *ptr, uint64_t rows, uint64_t cols, uint32_t box
     return m;
 }
 
+// One CTA an SM: 192 KB of operands in flight.
+constexpr int stages_for(int bn) { return bn == 256 ? 4 : bn == 128 ? 6 : 8; }
+
+template <int BN, int MODE>
+void allow_smem() {
+    static bool attr = false;  // one flag per instantiation
+    if (!attr) {
+        XG_CUDA(cudaFuncSetAttribute(k_gemm_bf16<BN, MODE>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                     192 * 1024 + 1024));
+        attr = true;
+    }
+}
+
+// CTAs of clusters of `split` that the GPU holds at once (a cluster lies within
+// one GPC, so this is fewer than one an SM).
+template <int BN>
+int query_cluster_ctas(int split, int sms) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)split * 64);
+    cfg.blockDim = dim3(THREADS);
+    cfg.dynamicSmemBytes = stages_for(BN) * stage_bytes(BN) + 1024;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)split;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    allow_smem<BN, F32>();
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16<BN, F32>, &cfg) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = std::max(1, sms / split / 2);
+    }
+    return n * split;
+}
+int cluster_ctas(int bn, int split, int sms) {
+    static int known[3][9] = {};
+    int &n = known[bn == 256 ? 2 : bn == 128 ? 1 : 0][split];
+    if (!n)
+        n = bn == 256   ? query_cluster_ctas<256>(split, sms)
+            : bn == 128 ? query_cluster_ctas<128>(split, sms)
+                        : query_cluster_ctas<64>(split, sms);
+    return n;
+}
+
 Shape shape_for(uint64_t M, uint64_t N, uint64_t K, int sms, bool may_split) {
     const uint64_t KB = K / BK;
     Shape best{128, 1, 6};
@@ -458,8 +506,9 @@ Shape shape_for(uint64_t M, uint64_t N, uint64_t K, int sms, bool may_split) {
         for (int split : {1, 2, 4, 8}) {
             if (split > 1 && (!may_split || KB < 4ull * split)) break;
             const uint64_t ctas = (M / BM) * (N / bn) * split;
-            consider(bn, split, bn == 256 ? 4 : bn == 128 ? 6 : 8,
-                     waves(ctas, sms) * ((double)((KB + split - 1) / split) * kb + T_FIXED +
+            consider(bn, split, stages_for(bn),
+                     waves(ctas, split > 1 ? cluster_ctas(bn, split, sms) : sms) *
+                         ((double)((KB + split - 1) / split) * kb + T_FIXED +
                                          (split > 1 ? T_SPLIT : 0.0)));
         }
         if (bn == 128)
@@ -474,12 +523,7 @@ void launch_mode(const CUtensorMap &ta, const CUtensorMap &tb, uint64_t M, uint6
     static_assert(BM * part_pitch(BN) * 4 <= 3 * stage_bytes(BN), "a tile fits in the stages");
     const uint32_t smem = (uint32_t)sh.stages * stage_bytes(BN) + 1024;  // + alignment slack
     auto kern = k_gemm_bf16<BN, MODE>;
-    static bool attr = false;  // one flag per instantiation
-    if (!attr) {
-        XG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     192 * 1024 + 1024));
-        attr = true;
-    }
+    allow_smem<BN, MODE>();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(N / BN) * (unsigned)sh.split, (unsigned)(M / BM));
     cfg.blockDim = dim3(THREADS);
