@@ -1332,11 +1332,31 @@ bool Krylov::persistent_ok() const {
     return ops::pbicgstab_persist_fits(*A, NV, cfg.gpu_persistent);
 }
 
+// The register-resident form's exchange buffer: zeroed when allocated, its tags
+// then grow from launch to launch. Returns its size (0: not that form).
+size_t Krylov::exchange_buffer(int sweeps) {
+    const size_t xb = ops::pbicgstab_exchange_bytes(*A, NV, sweeps, cfg.gpu_persistent);
+    if (xb > pexchange.bytes) {
+        pexchange.alloc(xb);
+        XG_CUDA(cudaMemsetAsync(pexchange.p, 0, xb, S()));
+    }
+    return xb;
+}
+
+// The persistent launch's buffers, where it will take the solves (allocated with
+// the solver; again only if renewed parameters ask for more).
+void Krylov::prepare_persistent() {
+    if (pcg || rbicgstab || !persistent_ok()) return;
+    if (!psync.bytes) psync.alloc(2 * sizeof(unsigned));
+    if (!pout.bytes) pout.alloc(128 * sizeof(double));
+    auto *jac = M ? dynamic_cast<Jacobi<double> *>(M.get()) : nullptr;
+    exchange_buffer(jac ? std::max(1, jac->cfg.max_iters) : 0);
+}
+
 void Krylov::run_persistent(DVec &x) {
     cudaStream_t s = S();
     auto *jac = M ? dynamic_cast<Jacobi<double> *>(M.get()) : nullptr;
-    if (!psync.bytes) psync.alloc(2 * sizeof(unsigned));
-    if (!pout.bytes) pout.alloc(128 * sizeof(double));
+    prepare_persistent();
     XG_CUDA(cudaMemsetAsync(psync.p, 0, psync.bytes, s));
     const k::RedArgs ra = ctx().red();
     k::PersistArgs P{};
@@ -1362,13 +1382,7 @@ void Krylov::run_persistent(DVec &x) {
     P.rel_tol = cfg.rel_tol;
     P.ra = ra;
     P.gs = k::GridSync{psync.as<unsigned long long>(), ra.flag, 1000000000ull};
-    // the register-resident form's exchange buffer: zeroed when allocated, its
-    // tags then grow from launch to launch
-    const size_t xb = ops::pbicgstab_exchange_bytes(*A, NV, P.sweeps, cfg.gpu_persistent);
-    if (xb > pexchange.bytes) {
-        pexchange.alloc(xb);
-        XG_CUDA(cudaMemsetAsync(pexchange.p, 0, xb, s));
-    }
+    const size_t xb = exchange_buffer(P.sweeps);
     ops::pbicgstab_persist(*A, P, NV, cfg.gpu_persistent, xb ? pexchange.p : nullptr,
                            ++plaunches << 36, s);
     double out[97];
@@ -1659,6 +1673,7 @@ void SolverHierarchy::build(const Params &P, const HCsr &hA_, const DCsr *A_, in
             kr->M = make_smoother(ic, "preconditioner", *A, hA, false, nv, 0, 0);
         }
         kr->enable_f32io();
+        kr->prepare_persistent();
         root.reset(kr);
         return;
     }

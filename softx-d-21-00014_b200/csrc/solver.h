@@ -109,6 +109,7 @@ class Krylov : public SolverBase {
     bool f32io_ready = false;  // pa32/sa32 allocated
     DVec pa32, sa32;
     void enable_f32io();
+    void prepare_persistent();  // its buffers, once M is known
     void setup() override;
     void solve(DVec &x, DVec &b, const std::vector<double> &conv) override;
     ~Krylov() override;
@@ -161,6 +162,7 @@ class Krylov : public SolverBase {
     // the whole iteration in one cooperative launch (k_pbicgstab_persist)
     bool persistent_ok() const;
     void run_persistent(DVec &x);
+    size_t exchange_buffer(int sweeps);
     DevBuf psync, pout;  // grid barrier counters; the launch's statistics
     DevBuf pexchange;    // exchange buffer of the register-resident form
     uint64_t plaunches = 0;  // its launches, the high bits of their tags
