@@ -205,29 +205,57 @@ struct Hsgs : public SolverBase {
         std::vector<uint64_t> off(nblocks + 1);
         for (int c = 0; c <= nblocks; ++c) off[c] = std::min<uint64_t>(n, cs * (uint64_t)c);
         off[nblocks] = n;
-        // block id of every row
-        std::vector<uint32_t> bid(n);
-        for (int c = 0; c < nblocks; ++c)
-            for (uint64_t i = off[c]; i < off[c + 1]; ++i) bid[i] = c;
+        // blocks are cs rows each, the last one short (split_range_f64); their
+        // rows padded to whole chunks (hsgs.cuh) where they fit in shared memory
+        auto block = [&](uint64_t i) { return std::min<uint64_t>(i / cs, (uint64_t)nblocks - 1); };
         HCsr dg, od;
         dg.nrows = od.nrows = n;
         od.ncols = n;
-        uint64_t maxb = 1;
-        for (int c = 0; c < nblocks; ++c) maxb = std::max<uint64_t>(maxb, off[c + 1] - off[c]);
-        dg.ncols = maxb;
         dg.row.assign(n + 1, 0);
         od.row.assign(n + 1, 0);
+        std::vector<uint32_t> in_block(n);
+        for (uint64_t i = 0; i < n; ++i) {
+            const uint64_t r0 = off[block(i)], r1 = off[block(i) + 1];
+            uint32_t in = 0;
+            for (uint64_t j = hA.row[i]; j < hA.row[i + 1]; ++j)
+                in += hA.col[j] >= r0 && hA.col[j] < r1;
+            in_block[i] = in;
+            od.row[i + 1] = od.row[i] + (hA.row[i + 1] - hA.row[i] - in);
+        }
+        auto chunked = [&](uint64_t i) {
+            return std::max<uint32_t>(4, (in_block[i] + 3) / 4 * 4);
+        };
+        plan.n = n;
+        plan.rows = (uint32_t)std::min<uint64_t>(cs, n);
+        for (int l = 0; l < 6; ++l) {
+            const uint64_t per = (uint64_t)plan.rows << l;
+            plan.ent_max[l] = 0;
+            for (uint64_t r = 0; r < n; r += per) {
+                uint32_t e = 0;
+                for (uint64_t i = r; i < std::min(n, r + per); ++i) e += chunked(i);
+                plan.ent_max[l] = std::max(plan.ent_max[l], e);
+            }
+        }
+        plan.padded = ops::hsgs_can_pad<F>(plan, NV);
+        for (uint64_t i = 0; i < n; ++i)
+            dg.row[i + 1] = dg.row[i] + (plan.padded ? chunked(i) : in_block[i]);
+        dg.ncols = (uint64_t)plan.rows + (plan.padded ? 1 : 0);
+        dg.col.assign(dg.row[n], plan.rows);  // padding entries: no row of the block
+        dg.val.assign(dg.row[n], 0.0);
+        od.col.resize(od.row[n]);
+        od.val.resize(od.row[n]);
         std::vector<std::pair<uint32_t, uint64_t>> tmp;
         for (uint64_t i = 0; i < n; ++i) {
-            const uint32_t c = bid[i];
+            const uint64_t r0 = off[block(i)], r1 = off[block(i) + 1];
+            uint32_t d0 = dg.row[i], o0 = od.row[i];
             tmp.clear();
             for (uint64_t j = hA.row[i]; j < hA.row[i + 1]; ++j) {
                 const uint32_t col = hA.col[j];
-                if (bid[col] == c) {
-                    dg.col.push_back((uint32_t)(col - off[c]));
-                    dg.val.push_back(hA.val[j]);
+                if (col >= r0 && col < r1) {
+                    dg.col[d0] = (uint32_t)(col - r0);
+                    dg.val[d0++] = hA.val[j];
                 } else {
-                    tmp.push_back({bid[col], j});
+                    tmp.push_back({(uint32_t)block(col), j});
                 }
             }
             // off-core chunks are visited in block order, entries in row order
@@ -235,44 +263,9 @@ struct Hsgs : public SolverBase {
                              [](const std::pair<uint32_t, uint64_t> &a,
                                 const std::pair<uint32_t, uint64_t> &b) { return a.first < b.first; });
             for (auto &t : tmp) {
-                od.col.push_back(hA.col[t.second]);
-                od.val.push_back(hA.val[t.second]);
+                od.col[o0] = hA.col[t.second];
+                od.val[o0++] = hA.val[t.second];
             }
-            dg.row[i + 1] = (uint32_t)dg.col.size();
-            od.row[i + 1] = (uint32_t)od.col.size();
-        }
-        // blocks are cs rows each, the last one short (split_range_f64); their
-        // rows padded to whole chunks (hsgs.cuh)
-        plan.n = n;
-        plan.rows = (uint32_t)std::min<uint64_t>(cs, n);
-        auto padded = [&](uint64_t i) {
-            const uint32_t len = dg.row[i + 1] - dg.row[i];
-            return std::max<uint32_t>(4, (len + 3) / 4 * 4);
-        };
-        for (int l = 0; l < 6; ++l) {
-            const uint64_t per = (uint64_t)plan.rows << l;
-            plan.ent_max[l] = 0;
-            for (uint64_t r = 0; r < n; r += per) {
-                uint32_t e = 0;
-                for (uint64_t i = r; i < std::min(n, r + per); ++i) e += padded(i);
-                plan.ent_max[l] = std::max(plan.ent_max[l], e);
-            }
-        }
-        plan.padded = ops::hsgs_can_pad<F>(plan, NV);
-        if (plan.padded) {
-            HCsr p;
-            p.nrows = n;
-            p.ncols = plan.rows + 1;
-            p.row.assign(n + 1, 0);
-            for (uint64_t i = 0; i < n; ++i) p.row[i + 1] = p.row[i] + padded(i);
-            p.col.assign(p.row[n], plan.rows);
-            p.val.assign(p.row[n], 0.0);
-            for (uint64_t i = 0; i < n; ++i)
-                for (uint64_t j = dg.row[i]; j < dg.row[i + 1]; ++j) {
-                    p.col[p.row[i] + (j - dg.row[i])] = dg.col[j];
-                    p.val[p.row[i] + (j - dg.row[i])] = dg.val[j];
-                }
-            std::swap(dg, p);
         }
         upload_csr(dg, Adiag, f32, cfg.gpu_index_compress, S());
         // absolute columns: a fused sweep reads off-block entries without their rows
