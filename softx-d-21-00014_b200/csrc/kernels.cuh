@@ -864,11 +864,15 @@ struct NoFin {
 };
 
 // What every SpMV epilogue shares: a row sum that starts from zero, and the
-// one-right-hand-side forms written with the vector ones. D is the epilogue,
+// one-right-hand-side forms written with the vector ones. (redirect, where there
+// are no dot products: the outputs go to scratch vectors a and b; the autotuner
+// times the very kernel that the solve launches.) D is the epilogue,
 // F its arithmetic type. Elements are indexed in 32 bits (the launchers check
 // that they fit).
 template <class D, typename F>
 struct EpiBase {
+    // bytes per value of the scratch vectors redirect() takes
+    static constexpr size_t SCRATCH_A = sizeof(F), SCRATCH_B = 0;
     __device__ F init(uint64_t, int) const { return F(0); }
     template <int VK, class P>
     __device__ void init(F (&y)[VK], const P &) const {
@@ -889,6 +893,7 @@ struct EStore : EpiBase<EStore<F, NV>, F>, NoFin {
     F *y;
     __host__ __device__ explicit EStore(F *y_) : y(y_) {}
     bool aligned() const { return aligned16(y); }
+    void redirect(void *a, void *) { y = (F *)a; }
     template <int VK>
     struct Pre {};
     template <int VK>
@@ -906,9 +911,11 @@ struct EStore : EpiBase<EStore<F, NV>, F>, NoFin {
 // y += A x  (csr_matvec.inl:106-120: accumulate directly into y)
 template <typename F, int NV>
 struct EAxpy : NoFin {
+    static constexpr size_t SCRATCH_A = sizeof(F), SCRATCH_B = 0;
     F *y;
     __host__ __device__ explicit EAxpy(F *y_) : y(y_) {}
     bool aligned() const { return aligned16(y); }
+    void redirect(void *a, void *) { y = (F *)a; }
     template <int VK>
     struct Pre {
         Vec<F, VK> y;
@@ -942,6 +949,7 @@ struct EResid : EpiBase<EResid<F, NV, NORM>, F> {
     double *out;  // NORM: sums land here (nv values)
     EResid(F *r_, const F *b_, double *out_) : r(r_), b(b_), out(out_) {}
     bool aligned() const { return aligned16(r) && aligned16(b); }
+    void redirect(void *a, void *) { r = (F *)a; }
     template <int VK>
     struct Pre {
         Vec<F, VK> b;
@@ -1097,6 +1105,7 @@ struct EJacobi : EpiBase<EJacobi<F, NV>, F>, NoFin {
     __host__ __device__ EJacobi(F *xout_, const F *xin_, const F *b_, const F *d_, F relax_)
         : xout(xout_), xin(xin_), b(b_), d(d_), relax(relax_) {}
     bool aligned() const { return aligned16(xout) && aligned16(xin) && aligned16(b); }
+    void redirect(void *a, void *) { xout = (F *)a; }
     template <int VK>
     struct Pre {
         Vec<F, VK> x, b;
@@ -1122,12 +1131,17 @@ struct EJacobi : EpiBase<EJacobi<F, NV>, F>, NoFin {
 // SpMV). x_zero: r = 1*b without the SpMV (used by k_rows through elem()).
 template <typename F, int NV>
 struct ECheby0 : EpiBase<ECheby0<F, NV>, F>, NoFin {
+    static constexpr size_t SCRATCH_B = sizeof(F);
     F *rs, *t1s;
     const F *b, *isd;
     F c;
     ECheby0(F *rs_, F *t1s_, const F *b_, const F *isd_, F c_)
         : rs(rs_), t1s(t1s_), b(b_), isd(isd_), c(c_) {}
     bool aligned() const { return aligned16(rs) && aligned16(t1s) && aligned16(b); }
+    void redirect(void *a, void *c2) {
+        rs = (F *)a;
+        t1s = (F *)c2;
+    }
     template <int VK>
     struct Pre {
         Vec<F, VK> b;
@@ -1220,6 +1234,7 @@ struct ECheby1 : EpiBase<ECheby1<F, NV>, F>, NoFin {
     ECheby1(F *out_, const F *rs_, const F *isd_, F c_, int last_, int x_zero_)
         : out(out_), rs(rs_), isd(isd_), c(c_), last(last_), x_zero(x_zero_) {}
     bool aligned() const { return aligned16(out) && aligned16(rs); }
+    void redirect(void *a, void *) { out = (F *)a; }
     template <int VK>
     struct Pre {
         Vec<F, VK> rs, x;
@@ -1258,10 +1273,12 @@ struct ECheby1 : EpiBase<ECheby1<F, NV>, F>, NoFin {
 // (x_zero: x = 1*t, the ax_y branch of axpby).
 template <int NV>
 struct EProlongMixed : EpiBase<EProlongMixed<NV>, float>, NoFin {
+    static constexpr size_t SCRATCH_A = sizeof(double);
     double *x;
     int x_zero;
     EProlongMixed(double *x_, int x_zero_) : x(x_), x_zero(x_zero_) {}
     bool aligned() const { return aligned16(x); }
+    void redirect(void *a, void *) { x = (double *)a; }
     template <int VK>
     struct Pre {
         Vec<double, VK> x;

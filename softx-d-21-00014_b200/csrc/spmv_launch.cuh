@@ -217,13 +217,26 @@ constexpr uint64_t WIDE_MAX_VALUES = 1u << 20;  // rows * nv up to which it is a
 // (1, 2, or none: tiles read from global memory, for small matrices where the
 // copy's round trip is not hidden) and the run of consecutive tiles a block
 // takes (1, 4 or 16, or the plane walk where the matrix has a walk stride) are
-// timed with CUDA events on the caller's x into a scratch y (EStore), once
-// per matrix, precision and nv, outside any graph capture; the fastest is
-// kept in the matrix (DCsr::tuned). Matrices of at most WIDE_MAX_VALUES rows
+// timed with CUDA events on the caller's x, with the epilogue of the call at hand
+// writing into scratch vectors, once per matrix, precision and nv, outside any
+// graph capture; the fastest is kept in the matrix (DCsr::tuned). (Timed as y = A
+// x, a Chebyshev step or a prolongation got the shape that is best without its
+// epilogue's operands: 34 us against 26 for the 96^3 prolongation.) Matrices of at most WIDE_MAX_VALUES rows
 // times nv also time the warp-per-row kernel (code TUNE_WIDE). Every candidate
 // sums each (row, right-hand side) in the same CSR order, so the choice never
 // changes a result.
 constexpr uint32_t TUNE_RUNS[3] = {1, 4, 16};
+// Scratch outputs of the timed launches of an epilogue (zeroed: some read what
+// they write).
+template <class Epi>
+struct TuneScratch {
+    DevBuf a, b;
+    TuneScratch(uint64_t values, cudaStream_t s)
+        : a(values * Epi::SCRATCH_A), b(values * Epi::SCRATCH_B) {
+        for (DevBuf *v : {&a, &b})
+            if (v->bytes) XG_CUDA(cudaMemsetAsync(v->p, 0, v->bytes, s));
+    }
+};
 struct Tuned {
     int alt;
     uint32_t nbuf, run;
@@ -252,15 +265,16 @@ constexpr int spmv_vk_alt() {
     return a <= NV ? a : d;
 }
 
-template <typename F, typename FX, typename I, int NV, typename V>
-static uint8_t autotune(const DCsr &A, const FX *x, cudaStream_t s) {
+template <typename F, typename FX, typename I, int NV, typename V, class Epi>
+static uint8_t autotune(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     XG_CUDA(cudaStreamIsCapturing(s, &cs));
     if (cs != cudaStreamCaptureStatusNone) return 0;
     constexpr int VD = k::spmv_vk<FX, NV>();
     constexpr int VA = spmv_vk_alt<FX, NV>();
-    DevBuf y(A.nrows * (uint64_t)NV * sizeof(F));
-    k::EStore<F, NV> e(y.as<F>());
+    TuneScratch<Epi> scratch(A.nrows * (uint64_t)NV, s);
+    Epi e = epi;
+    e.redirect(scratch.a.p, scratch.b.p);
     cudaEvent_t e0, e1;
     XG_CUDA(cudaEventCreate(&e0));
     XG_CUDA(cudaEventCreate(&e1));
@@ -366,7 +380,7 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
             int l = 0;
             while ((1 << l) < NV) ++l;
             uint8_t &t = A.tuned[sizeof(F) == 4][sizeof(FX) == 4][l];
-            if (!t) t = autotune<F, FX, I, NV, V>(A, x, s);
+            if (!t) t = autotune<F, FX, I, NV, V>(A, x, epi, s);
             if (t == TUNE_WIDE) {
                 launch_wide<F, FX, I, NV, V>(A, x, epi, s);
                 return;
@@ -469,23 +483,24 @@ static void launch_stencil(const DCsr &A, const F *x, const Epi &epi, cudaStream
 
 // Stencil or CSR (DCsr::st_choice): on matrices with a grid-stencil copy and
 // tuning on, the first SpMV without dot products for each precision and nv
-// times y = A x (EStore into a scratch y, the caller's x) with the stencil
+// times the call at hand (its outputs into scratch vectors) with the stencil
 // kernel's two register budgets and with the CSR kernel's tuned shape (the
 // faster of two rounds of three launches each, outside any graph capture).
 // A stencil form is kept only when it is at least ST_MARGIN faster than the
-// CSR kernel: the smoothers' epilogues read and write more vectors than the
-// timed y = A x, which costs the register-heavy stencil kernel more
-// (measured in the 128^3 solve: its Chebyshev steps 13 % slower than CSR at
-// equal y = A x times). All give the same results bit for bit.
+// CSR kernel: the level's other epilogues may read and write more vectors than
+// the timed one, which costs the register-heavy stencil kernel more (measured in
+// the 128^3 solve: its Chebyshev steps 13 % slower than CSR at equal y = A x
+// times). All give the same results bit for bit.
 constexpr float ST_MARGIN = 0.9f;
 constexpr uint8_t ST_USE64 = 1, ST_USE128 = 2, ST_USE_CSR = 3;
-template <typename F, typename I, int NV, bool CALLER_X>
-static uint8_t tune_stencil(const DCsr &A, const F *x, cudaStream_t s) {
+template <typename F, typename I, int NV, bool CALLER_X, class Epi>
+static uint8_t tune_stencil(const DCsr &A, const F *x, const Epi &epi, cudaStream_t s) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     XG_CUDA(cudaStreamIsCapturing(s, &cs));
     if (cs != cudaStreamCaptureStatusNone) return 0;
-    DevBuf y(A.nrows * (uint64_t)NV * sizeof(F));
-    k::EStore<F, NV> e(y.as<F>());
+    TuneScratch<Epi> scratch(A.nrows * (uint64_t)NV, s);
+    Epi e = epi;
+    e.redirect(scratch.a.p, scratch.b.p);
     cudaEvent_t e0, e1;
     XG_CUDA(cudaEventCreate(&e0));
     XG_CUDA(cudaEventCreate(&e1));
@@ -548,7 +563,7 @@ static void launch(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s) {
                 int l = 0;
                 while ((1 << l) < NV) ++l;
                 uint8_t &c = A.st_choice[sizeof(F) == 4][l];
-                if (!c) c = tune_stencil<F, I, NV, CALLER_X>(A, x, s);
+                if (!c) c = tune_stencil<F, I, NV, CALLER_X>(A, x, epi, s);
                 if (c) choice = c;
             }
             if (choice != ST_USE_CSR) {
