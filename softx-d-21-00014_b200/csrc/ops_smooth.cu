@@ -104,7 +104,16 @@ template void hsgs_sweep<float>(const DCsr &, const HsgsPlan &, const uint64_t *
 
 // The fused form needs one-byte in-block columns (blocks of at most 254 rows,
 // narrowed), absolute off-block columns and a block that fits beside the
-// products; x offsets are formed in 32 bits.
+// products; x offsets are formed in 32 bits. It saves a launch and the lagged
+// term's way through memory (8-9 us on small levels), and costs 2-3 ns for each
+// off-block product of a thread block, of which the sweep's registers let four
+// share an SM. So it is taken where the thread blocks fit the GPU at once and
+// form at most 4096 products each. Sweep, fused against SpMV + sweep (us, FP32):
+// 56^3 nv = 1 second level (1.4 K products) 18 against 22; 88^3 nv = 4 third
+// level (6.4 K) 35 against 27, finest level (2130 thread blocks) 94 against 59;
+// 96^3 nv = 16 finest level 353 against 234, second level 284 against 117.
+constexpr uint64_t HS_FUSE_PRODUCTS = 4096;
+constexpr int HS_FUSE_BLOCKS = 4;
 template <typename F>
 bool hsgs_can_fuse(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, int nv) {
     if (Adiag.col_bytes != 1 || Aoff.col_bytes < 0 || Adiag.nrows == 0) return false;
@@ -112,7 +121,11 @@ bool hsgs_can_fuse(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, in
     bool ok = false;
     dispatch_nv(nv, [&](auto nvc) {
         k::HsgsShape sh;
-        ok = hsgs_shape<F, decltype(nvc)::value>(plan, true, sh);
+        if (!hsgs_shape<F, decltype(nvc)::value>(plan, true, sh)) return;
+        const uint64_t per = (uint64_t)plan.rows * sh.group;
+        const uint64_t blocks = (Adiag.nrows + per - 1) / per;
+        ok = blocks <= (uint64_t)HS_FUSE_BLOCKS * (uint64_t)ctx().sms &&
+             Aoff.nnz * (uint64_t)nv <= HS_FUSE_PRODUCTS * blocks;
     });
     return ok;
 }
