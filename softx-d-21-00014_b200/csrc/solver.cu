@@ -372,9 +372,6 @@ struct Chebyshev : public SolverBase {
     DevBuf isd;
     double min_eig = 0, max_eig = 0;
     std::vector<F> coef;
-    // set by the multigrid for its next call: the input b is still in double
-    // here and is rounded into b by the first step (x zero-flagged)
-    const double *from64 = nullptr;
     void setup_from(const HCsr &hA) {
         if (f32)
             upload(isd, inv_diag_f32(hA, true), S());
@@ -384,6 +381,11 @@ struct Chebyshev : public SolverBase {
         XG_CUDA(cudaStreamSynchronize(S()));
     }
     void solve(DVec &x, DVec &b, const std::vector<double> &conv) override {
+        apply(x, b, conv, nullptr);
+    }
+    // b64 (x zero-flagged): the input is still in double there, and the first
+    // step rounds it into b
+    void apply(DVec &x, DVec &b, const std::vector<double> &conv, const double *b64) {
         reset_stats();
         const int order = cfg.poly_order;
         XG_REQUIRE(order >= 1 && order <= 4, XAMG_ERR_INVALID_ARG,
@@ -400,8 +402,6 @@ struct Chebyshev : public SolverBase {
         }
         DVec &rs = buf[0];
         DVec *t1s = &buf[1], *other = &buf[2];
-        const double *b64 = from64;
-        from64 = nullptr;
         if constexpr (std::is_same<F, float>::value) {
             if (b64)
                 ops::cheby_first_from64(n, b64, b.p<float>(), isd.as<float>(), coef[order - 1],
@@ -668,15 +668,19 @@ void MultiGrid::build(const HCsr &A0, const DCsr *A0dev, const Params &P, const 
     XG_CUDA(cudaStreamSynchronize(S()));
 }
 
-// mg.inl:166-260
-void MultiGrid::cycle(int level, DVec &x, DVec &b, int cyc, const std::vector<double> &iconv) {
+// mg.inl:166-260; b64: take_input's result (level 0)
+void MultiGrid::cycle(int level, DVec &x, DVec &b, int cyc, const std::vector<double> &iconv,
+                      const double *b64) {
     MgLevel &lv = L[level];
     const DCsr &Al = (level == 0 && !full32) ? *A : lv.A;
     const int nl = (int)L.size();
     MgLevel &nx = L[level + 1];
     DVec &temp = lv.temp, &bH = nx.bH, &xH = nx.xH;
     const bool mixed = (lv.f32 != nx.f32);  // level 0 -> 1 with reduced precision
-    if (cyc != 1) pre[level]->solve(x, b, iconv);
+    if (b64)
+        static_cast<Chebyshev<float> *>(pre[level].get())->apply(x, b, iconv, b64);
+    else if (cyc != 1)
+        pre[level]->solve(x, b, iconv);
     // residual temp = b - A x (Ax_y + axpby(a1, b, a_1, temp))
     const DVec *rin = &temp;
     if (x.zero) {
@@ -733,18 +737,18 @@ void MultiGrid::cycle(int level, DVec &x, DVec &b, int cyc, const std::vector<do
     post[level]->solve(x, b, iconv);
 }
 
-// Rounds the preconditioner's double input b into b32, or leaves that to the
-// first step of the finest level's Chebyshev pre-smoother where the cycle
-// starts with it from x = 0.
-void MultiGrid::take_input(DVec &b, bool x_zero) {
+// Rounds the preconditioner's double input b into b32 (null), or, where the
+// cycle starts from x = 0 with the finest level's Chebyshev pre-smoother, leaves
+// that to the smoother's first step: returns the input that the first cycle hands it.
+const double *MultiGrid::take_input(DVec &b, bool x_zero) {
     b32.zero = b.zero;
     b32.init = true;
-    if (b.zero) return;
+    if (b.zero) return nullptr;
     auto *ch = dynamic_cast<Chebyshev<float> *>(pre[0].get());
     if (ch && x_zero && cfg.mg_cycle != 1 && !(ch->cfg.convergence_check && ch->cfg.convergence_info))
-        ch->from64 = b.p<double>();
-    else
-        ops::convert<float, double>(b32.p<float>(), b.p<double>(), b.elems(), S());
+        return b.p<double>();
+    ops::convert<float, double>(b32.p<float>(), b.p<double>(), b.elems(), S());
+    return nullptr;
 }
 
 // The gpu_precond_f32 = 1 preconditioner with its result left in float in
@@ -753,11 +757,12 @@ void MultiGrid::take_input(DVec &b, bool x_zero) {
 void MultiGrid::solve_to32(DVec &x32o, DVec &b, const std::vector<double> &conv) {
     reset_stats();
     std::vector<double> iconv = conv;
-    take_input(b, x32o.zero);
+    const double *b64 = take_input(b, x32o.zero);
     x32o.init = true;
     do {
         ++st.iters;
-        cycle(0, x32o, b32, cfg.mg_cycle, iconv);
+        cycle(0, x32o, b32, cfg.mg_cycle, iconv, b64);
+        b64 = nullptr;
     } while (st.iters < cfg.max_iters);
 }
 
@@ -769,13 +774,14 @@ void MultiGrid::solve(DVec &x, DVec &b, const std::vector<double> &conv) {
     if (full32) {
         // preconditioner in float throughout: convert the input, cycle, convert
         // the result back (zero flags carried across)
-        take_input(b, x.zero);
+        const double *b64 = take_input(b, x.zero);
         x32.zero = x.zero;
         if (!x.zero) ops::convert<float, double>(x32.p<float>(), x.p<double>(), x.elems(), S());
         x32.init = true;
         do {
             ++st.iters;
-            cycle(0, x32, b32, cfg.mg_cycle, iconv);
+            cycle(0, x32, b32, cfg.mg_cycle, iconv, b64);
+            b64 = nullptr;
         } while (st.iters < cfg.max_iters);
         x.zero = x32.zero;
         if (!x32.zero) ops::convert<double, float>(x.p<double>(), x32.p<float>(), x.elems(), S());

@@ -79,8 +79,9 @@ class MultiGrid : public SolverBase {
     void solve_to32(DVec &x32, DVec &b, const std::vector<double> &conv);
 
   private:
-    void cycle(int level, DVec &x, DVec &b, int cyc, const std::vector<double> &iconv);
-    void take_input(DVec &b, bool x_zero);
+    void cycle(int level, DVec &x, DVec &b, int cyc, const std::vector<double> &iconv,
+               const double *b64 = nullptr);
+    const double *take_input(DVec &b, bool x_zero);
 };
 
 // A preconditioner application captured as a CUDA graph: the kernels that
