@@ -158,6 +158,12 @@ int XAMG_b200_solver_level_info(size_t sid, int level, int which, uint64_t *nrow
  * bit for bit. */
 int XAMG_b200_solver_level_tuned(size_t sid, int level, int which, uint8_t *codes);
 
+/* The Gauss-Seidel pre-smoother of a level (no counterpart): the stored column
+ * width of its off-block entries (as col_bytes in XAMG_b200_csr; 0: the level's
+ * pre-smoother is another one) and whether the sweep forms the lagged term of
+ * those entries itself (small levels) or a SpMV before it does. */
+int XAMG_b200_solver_level_hsgs(size_t sid, int level, int *off_col_bytes, int *fused);
+
 /* Grid-stencil storage (parameter gpu_index_compress = 3; no counterpart in
  * the reference, whose CSR blocks always carry column indices). A square
  * matrix whose entries all lie on the offsets dz*S2 + dy*S + dx (|dz|, |dy|,

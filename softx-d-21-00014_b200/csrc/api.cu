@@ -931,6 +931,19 @@ int XAMG_b200_solver_level_tuned(size_t sid, int level, int which, uint8_t *code
     });
 }
 
+int XAMG_b200_solver_level_hsgs(size_t sid, int level, int *off_col_bytes, int *fused) {
+    return guarded([&] {
+        XG_REQUIRE(off_col_bytes && fused, XAMG_ERR_INVALID_ARG, "null pointer");
+        MultiGrid *mg = solver_mg(sid);
+        XG_REQUIRE(mg && level >= 0 && level < (int)mg->pre.size(), XAMG_ERR_INVALID_ARG,
+                   "no smoother on that level");
+        bool f = false;
+        const DCsr *off = mg->pre[level]->off_block(f);
+        *off_col_bytes = off ? off->col_bytes : 0;
+        *fused = f ? 1 : 0;
+    });
+}
+
 int XAMG_b200_solver_level_download(size_t sid, int level, int which, uint32_t *row, void *col,
                                     void *val) {
     return guarded([&] {

@@ -151,9 +151,10 @@ void hsgs_sweep(const DCsr &Adiag, const HsgsPlan &plan, const uint64_t *boff, i
                 cudaStream_t s);
 
 // The same sweep with its lagged term b - A_offblock xin formed inside, into
-// another vector than xin; hsgs_can_fuse: whether the blocks allow it.
+// another vector than xin; Aoff's columns are absolute. hsgs_can_fuse: whether
+// the blocks allow it, from the off-block entry count (Aoff is uploaded after).
 template <typename F>
-bool hsgs_can_fuse(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, int nv);
+bool hsgs_can_fuse(const DCsr &Adiag, uint64_t off_nnz, const HsgsPlan &plan, int nv);
 template <typename F>
 void hsgs_fused_sweep(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, const F *b,
                       const F *xin, F *xout, const F *d, const double *relax_sc, int nv,

@@ -115,8 +115,8 @@ template void hsgs_sweep<float>(const DCsr &, const HsgsPlan &, const uint64_t *
 constexpr uint64_t HS_FUSE_PRODUCTS = 4096;
 constexpr int HS_FUSE_BLOCKS = 4;
 template <typename F>
-bool hsgs_can_fuse(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, int nv) {
-    if (Adiag.col_bytes != 1 || Aoff.col_bytes < 0 || Adiag.nrows == 0) return false;
+bool hsgs_can_fuse(const DCsr &Adiag, uint64_t off_nnz, const HsgsPlan &plan, int nv) {
+    if (Adiag.col_bytes != 1 || Adiag.nrows == 0) return false;
     if (Adiag.nrows * (uint64_t)nv >= (1ull << 32)) return false;
     bool ok = false;
     dispatch_nv(nv, [&](auto nvc) {
@@ -125,12 +125,12 @@ bool hsgs_can_fuse(const DCsr &Adiag, const DCsr &Aoff, const HsgsPlan &plan, in
         const uint64_t per = (uint64_t)plan.rows * sh.group;
         const uint64_t blocks = (Adiag.nrows + per - 1) / per;
         ok = blocks <= (uint64_t)HS_FUSE_BLOCKS * (uint64_t)ctx().sms &&
-             Aoff.nnz * (uint64_t)nv <= HS_FUSE_PRODUCTS * blocks;
+             off_nnz * (uint64_t)nv <= HS_FUSE_PRODUCTS * blocks;
     });
     return ok;
 }
-template bool hsgs_can_fuse<double>(const DCsr &, const DCsr &, const HsgsPlan &, int);
-template bool hsgs_can_fuse<float>(const DCsr &, const DCsr &, const HsgsPlan &, int);
+template bool hsgs_can_fuse<double>(const DCsr &, uint64_t, const HsgsPlan &, int);
+template bool hsgs_can_fuse<float>(const DCsr &, uint64_t, const HsgsPlan &, int);
 
 template <typename F>
 void hsgs_fused_sweep(const DCsr &A, const DCsr &Aoff, const HsgsPlan &plan, const F *b,

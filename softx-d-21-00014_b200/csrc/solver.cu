@@ -268,9 +268,10 @@ struct Hsgs : public SolverBase {
             }
         }
         upload_csr(dg, Adiag, f32, cfg.gpu_index_compress, S());
-        // absolute columns: a fused sweep reads off-block entries without their rows
-        upload_csr(od, Aoff, f32, std::min(cfg.gpu_index_compress, 1), S(), cfg.gpu_spmv_tune);
-        fuse = ops::hsgs_can_fuse<F>(Adiag, Aoff, plan, NV);
+        // a fused sweep reads off-block entries without their rows: absolute columns
+        fuse = ops::hsgs_can_fuse<F>(Adiag, od.nnz(), plan, NV);
+        upload_csr(od, Aoff, f32, fuse ? std::min(cfg.gpu_index_compress, 1) : cfg.gpu_index_compress,
+                   S(), cfg.gpu_spmv_tune);
         upload(boff, off, S());
         if (f32)
             upload(d, inv_diag_f32(hA, false), S());
@@ -282,6 +283,10 @@ struct Hsgs : public SolverBase {
                                 cudaMemcpyHostToDevice, S()));
         alloc_buffers(2);
         XG_CUDA(cudaStreamSynchronize(S()));
+    }
+    const DCsr *off_block(bool &fused) const override {
+        fused = fuse;
+        return &Aoff;
     }
     // The sweeps without a convergence test: x alternates between x and
     // buf[1], sweep j landing in x when (m - j) is even so that the last one

@@ -37,6 +37,12 @@ struct SolverBase {
     virtual void setup() {}
     // conv: NV entries, 1 = still active, 0 = converged (the "iconv" vector)
     virtual void solve(DVec &x, DVec &b, const std::vector<double> &conv) = 0;
+    // Gauss-Seidel smoothers: the operator of the lagged term, and whether the
+    // sweep forms that term itself
+    virtual const DCsr *off_block(bool &fused) const {
+        fused = false;
+        return nullptr;
+    }
     void reset_stats();
     void alloc_buffers(int count);
 };

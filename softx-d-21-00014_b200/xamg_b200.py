@@ -62,7 +62,7 @@ EXT_SYMBOLS = [
     "XAMG_b200_mlp_destroy", "XAMG_b200_mlp_predict", "XAMG_b200_mlp_train_step",
     "XAMG_b200_mlp_gradients", "XAMG_b200_mlp_params", "XAMG_b200_solver_solve_batch",
     "XAMG_b200_solver_level_tuned", "XAMG_b200_stencil_layout", "XAMG_b200_solver_level_stencil",
-    "XAMG_b200_solver_level_xstaged",
+    "XAMG_b200_solver_level_xstaged", "XAMG_b200_solver_level_hsgs",
 ]
 
 
@@ -204,6 +204,8 @@ def lib():
         "XAMG_b200_solver_level_tuned": (C.c_int, [C.c_size_t, C.c_int, C.c_int, vp]),
         "XAMG_b200_solver_level_xstaged": (C.c_int, [C.c_size_t, C.c_int, C.c_int,
                                                      C.POINTER(C.c_int)]),
+        "XAMG_b200_solver_level_hsgs": (C.c_int, [C.c_size_t, C.c_int, C.POINTER(C.c_int),
+                                                  C.POINTER(C.c_int)]),
         "XAMG_b200_stencil_layout": (C.c_int, [u64, vp, vp, C.POINTER(C.c_int),
                                                C.POINTER(C.c_uint32), C.POINTER(C.c_uint32),
                                                C.POINTER(C.c_int)]),
@@ -541,6 +543,13 @@ class Solver:
         v = C.c_int()
         call("XAMG_b200_solver_level_xstaged", self.h, level, which, C.byref(v))
         return v.value
+
+    def level_hsgs(self, level):
+        """The level's Gauss-Seidel pre-smoother: (column width of its off-block
+        entries, whether the sweep forms their lagged term itself)."""
+        w, f = C.c_int(), C.c_int()
+        call("XAMG_b200_solver_level_hsgs", self.h, level, C.byref(w), C.byref(f))
+        return w.value, bool(f.value)
 
     def level_stencil(self, level, which):
         """The level matrix's grid-stencil copy: (pattern, S, S2, diag_first),

@@ -28,3 +28,23 @@ def test_hsgs_forms(gpu, oracle, nv, rows, sweeps, reduced, narrow):
               "coarse_grid_solver": {"method": "Direct"}}
     st, _ = check(gpu, oracle, row, col, val, nv, params, seed=nv + rows, hsgs_rows=rows)
     assert st["conv"].all()
+
+
+@pytest.mark.parametrize("nv,off", [(8, (-2, False)), (1, (4, True))])
+def test_off_block_columns(gpu, oracle, nv, off):
+    """Two-byte relative columns (gpu_index_compress = 2) of a level of more than
+    65,536 rows whose lagged term stays a SpMV; absolute ones where the sweep
+    forms it."""
+    row, col, val = gpu.generate_diffusion(7, 41, 41, 41, 1.0, 1.0, 3)
+    sm = {"method": "HSGS", "max_iters": 1}
+    params = {"solver": {"method": "MergedPBiCGStab", "max_iters": 100, "rel_tolerance": 1e-8,
+                         "abs_tolerance": 0, "gpu_index_compress": 2},
+              "preconditioner": dict(MG_BASE, method="MultiGrid", gpu_precond_f32=1,
+                                     gpu_index_compress=2, mg_coarse_matrix_size=500),
+              "pre_smoother": sm, "post_smoother": dict(sm),
+              "coarse_grid_solver": {"method": "Direct"}}
+    st, S = check(gpu, oracle, row, col, val, nv, params, seed=1)
+    assert st["conv"].all()
+    assert S.level_hsgs(0) == off
+    # at most 65,536 columns on the coarser levels
+    assert all(S.level_hsgs(lv)[0] in (1, 2) for lv in range(1, S.nlevels() - 1))
