@@ -158,16 +158,13 @@ struct Epilogue {
     bool aux_vec;        // four values of aux at once are aligned
 };
 
-// What the epilogue of four consecutive columns n.. of one row reads.
+// What the epilogue of four consecutive columns n.. of one row reads beside the
+// bias.
 struct Operands {
-    float b[4], t[4];
+    float t[4];
 };
 template <int MODE>
 __device__ __forceinline__ void operands(Operands &o, const Epilogue &ep, uint64_t row, int n) {
-    if (MODE != BF16_MASK && ep.bias) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) o.b[i] = __ldg(&ep.bias[n + i]);
-    }
     if constexpr (MODE == MSE_GRAD) {
         const float *t = (const float *)ep.aux + row * ep.ld_aux + n;
         if (ep.aux_vec) {
@@ -192,13 +189,13 @@ __device__ __forceinline__ void operands(Operands &o, const Epilogue &ep, uint64
 }
 // Returns the squared errors of the four values (MSE_GRAD).
 template <int MODE>
-__device__ __forceinline__ double finish(const Operands &o, const Epilogue &ep, uint64_t row, int n,
-                                         float4 acc) {
+__device__ __forceinline__ double finish(const Operands &o, const float (&bias)[4],
+                                         const Epilogue &ep, uint64_t row, int n, float4 acc) {
     float v[4] = {acc.x, acc.y, acc.z, acc.w};
     double sq = 0.0;
     if (MODE != BF16_MASK && ep.bias) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) v[i] += o.b[i];
+        for (int i = 0; i < 4; ++i) v[i] += bias[i];
     }
     if constexpr (MODE == F32) {
         *(float4 *)((float *)ep.C + row * ep.ldc + n) = make_float4(v[0], v[1], v[2], v[3]);
@@ -261,18 +258,33 @@ __global__ void __launch_bounds__(THREADS, 2)
     const uint32_t tmem = tmem_holder;
     bool ok = true;
     double sq = 0.0;
+    // The epilogue's columns of this thread, the same in every row it takes, and
+    // their bias, on its way during the main loop: read again for every row it took
+    // 2 us of a BF16 tile of 128 columns.
+    constexpr int Q = BN / 4;
+    static_assert(THREADS % Q == 0, "a thread keeps its columns");
+    const int col = (int)(threadIdx.x % Q) * 4, n = n0 + col;
+    float bias[4];
+    if (MODE != BF16_MASK && ep.bias) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) bias[i] = __ldg(&ep.bias[n + i]);
+    }
 
+    // The two threads of the main loop count stage, parity, addresses and descriptors
+    // up: with a division by the number of stages and each descriptor formed anew, a
+    // k-block took 0.385 us instead of 0.31 whatever the tile's width (one B200).
     if (warp == 0 && lane == 0) {
         // producer: TMA loads of the k-blocks into the stage ring
-        int issued = 0;
-        for (int i = 0; i < nkb && ok; ++i) {
-            const int s = i % stages;
-            const uint32_t u = (uint32_t)(i / stages);
-            if (i >= stages && !k::mbar_wait(&empty[s], (u - 1) & 1u)) ok = false;
-            if (!ok) break;
+        int issued = 0, s = 0, kx = kb0 * BK;
+        uint32_t parity = 1;  // of the stage's last release
+        unsigned char *a = smem;
+        for (; issued < nkb; ++issued) {
+            if (issued >= stages && !k::mbar_wait(&empty[s], parity)) {
+                ok = false;
+                break;
+            }
             k::mbar_arrive_expect(&full[s], STAGE);
-            unsigned char *a = smem + (size_t)s * STAGE, *b = a + TILE_A;
-            const int kx = (kb0 + i) * BK;
+            unsigned char *b = a + TILE_A;
             if (a_mn) {
                 for (int j = 0; j < BM / 64; ++j)
                     tma_load_2d(a + j * BOX, &ta, m0 + j * 64, kx, &full[s]);
@@ -285,28 +297,44 @@ __global__ void __launch_bounds__(THREADS, 2)
             } else {
                 tma_load_2d(b, &tb, kx, n0, &full[s]);
             }
-            ++issued;
+            kx += BK;
+            a += STAGE;
+            if (++s == stages) {
+                s = 0;
+                a = smem;
+                parity ^= 1u;
+            }
         }
         if (!ok)  // no exit with a copy into this CTA's shared memory in flight
             for (int i = issued > stages ? issued - stages : 0; i < issued; ++i)
                 k::mbar_wait(&full[i % stages], (uint32_t)(i / stages) & 1u);
     } else if (warp == 1 && lane == 0) {
-        // MMA issuer: four K = 16 steps per stage, then release the stage
+        // MMA issuer: four K = 16 steps per stage, then release the stage. The
+        // descriptors differ in their start address only, in 16-byte units.
         const uint32_t id = idesc(BN, a_mn, b_mn);
-        const uint32_t sa = a_mn ? 2048u : 32u, sb = b_mn ? 2048u : 32u;
+        const uint32_t sa = (a_mn ? 2048u : 32u) >> 4, sb = (b_mn ? 2048u : 32u) >> 4;
+        const uint64_t a0 = sw128_desc(saddr(smem), a_mn), b0 = sw128_desc(saddr(smem) + TILE_A, b_mn);
+        uint64_t da = a0, db = b0;
+        int s = 0;
+        uint32_t parity = 0;
         for (int i = 0; i < nkb; ++i) {
-            const int s = i % stages;
-            if (!k::mbar_wait(&full[s], (uint32_t)(i / stages) & 1u)) {
+            if (!k::mbar_wait(&full[s], parity)) {
                 ok = false;
                 break;
             }
             tc_fence_after();
-            const uint32_t a = saddr(smem + (size_t)s * STAGE), b = a + TILE_A;
 #pragma unroll
             for (int kk = 0; kk < BK / 16; ++kk)
-                mma_bf16(tmem, sw128_desc(a + kk * sa, a_mn), sw128_desc(b + kk * sb, b_mn), id,
-                         (i | kk) != 0);
+                mma_bf16(tmem, da + kk * sa, db + kk * sb, id, (i | kk) != 0);
             mma_commit(&empty[s]);
+            da += STAGE >> 4;
+            db += STAGE >> 4;
+            if (++s == stages) {
+                s = 0;
+                da = a0;
+                db = b0;
+                parity ^= 1u;
+            }
         }
         mma_commit(&acc_full);  // arrives once every MMA issued above has completed
     } else if (warp >= 2) {
@@ -332,23 +360,22 @@ __global__ void __launch_bounds__(THREADS, 2)
     if (split == 1) {
         __syncthreads();  // the tile is written
         const float *part = (const float *)smem;
-        constexpr int Q = BN / 4, STEPS = (BM * Q + THREADS - 1) / THREADS;
+        constexpr int RT = THREADS / Q, STEPS = (BM + RT - 1) / RT;  // rows at a time
+        const int r0 = (int)threadIdx.x / Q;
 #pragma unroll 1
         for (int s0 = 0; s0 < STEPS; s0 += 4) {  // four rows' operands in flight
             Operands o[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int t = (s0 + u) * THREADS + threadIdx.x;
-                if (t < BM * Q)
-                    operands<MODE>(o[u], ep, (uint64_t)m0 + t / Q, n0 + (t % Q) * 4);
+                const int r = (s0 + u) * RT + r0;
+                if (r < BM) operands<MODE>(o[u], ep, (uint64_t)m0 + r, n);
             }
 #pragma unroll
             for (int u = 0; u < 4; ++u) {
-                const int t = (s0 + u) * THREADS + threadIdx.x;
-                if (t < BM * Q)
-                    sq += finish<MODE>(o[u], ep, (uint64_t)m0 + t / Q, n0 + (t % Q) * 4,
-                                       *(const float4 *)(part + t / Q * part_pitch(BN) +
-                                                         (t % Q) * 4));
+                const int r = (s0 + u) * RT + r0;
+                if (r < BM)
+                    sq += finish<MODE>(o[u], bias, ep, (uint64_t)m0 + r, n,
+                                       *(const float4 *)(part + r * part_pitch(BN) + col));
             }
         }
     } else {
@@ -356,11 +383,11 @@ __global__ void __launch_bounds__(THREADS, 2)
         cluster_sync();  // every CTA's partial tile is written
         const int rows = BM / split;
         const uint32_t base = saddr(smem);
-        for (int t = threadIdx.x; t < rows * (BN / 4); t += THREADS) {
-            const int r = rank * rows + t / (BN / 4), c = (t % (BN / 4)) * 4;
-            const uint32_t off = (uint32_t)(r * part_pitch(BN) + c) * 4;
+        for (int t = threadIdx.x; t < rows * Q; t += THREADS) {
+            const int r = rank * rows + t / Q;
+            const uint32_t off = (uint32_t)(r * part_pitch(BN) + col) * 4;
             Operands o;
-            operands<MODE>(o, ep, (uint64_t)m0 + r, n0 + c);
+            operands<MODE>(o, ep, (uint64_t)m0 + r, n);
             float4 p[8];
 #pragma unroll
             for (int s = 0; s < 8; ++s)  // all in flight
@@ -374,7 +401,7 @@ __global__ void __launch_bounds__(THREADS, 2)
                     v.z += p[s].z;
                     v.w += p[s].w;
                 }
-            sq += finish<MODE>(o, ep, (uint64_t)m0 + r, n0 + c, v);
+            sq += finish<MODE>(o, bias, ep, (uint64_t)m0 + r, n, v);
         }
     }
     if constexpr (MODE == MSE_GRAD) {
