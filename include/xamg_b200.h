@@ -244,6 +244,17 @@ int XAMG_b200_gemm_bf16(uint64_t M, uint64_t N, uint64_t K, const void *A, const
                         void *C, uint64_t ldc, int mode, const float *bias, const void *aux,
                         uint64_t ld_aux, void *stream);
 
+/* The tile width, K split and pipeline stages such a GEMM takes (no
+ * counterpart): shape[0..2]. may_split: the sum over K may be split between the
+ * CTAs of a cluster, as XAMG_b200_gemm_bf16 does (the MLP's training products do
+ * not). transposed: both operands are stored transposed, as in the MLP's weight
+ * gradients. cluster_ctas, if not NULL, describes a GPU of `sms` multiprocessors by the
+ * CTAs it holds at once for each tile width (64, 128, 256) and split (1, 2, 4, 8;
+ * 0: none), 12 values: the rule then runs on the host alone. NULL: the GPU in use
+ * (sms ignored). */
+int XAMG_b200_gemm_shape(uint64_t M, uint64_t N, uint64_t K, int may_split, int transposed,
+                         int sms, const int *cluster_ctas, int *shape);
+
 /* The MLP of the learned coarse initial guess (no counterpart): n_in -> h ->
  * h -> n_out dense layers with ReLU, BF16 weights and activations on the
  * tcgen05 GEMM with FP32 accumulation, FP32 master weights trained by Adam on

@@ -1043,6 +1043,26 @@ int XAMG_b200_gemm_bf16(uint64_t M, uint64_t N, uint64_t K, const void *A, const
     });
 }
 
+int XAMG_b200_gemm_shape(uint64_t M, uint64_t N, uint64_t K, int may_split, int transposed,
+                         int sms, const int *cluster_ctas, int *shape) {
+    return guarded([&] {
+        XG_REQUIRE(shape && (!cluster_ctas || sms > 0), XAMG_ERR_INVALID_ARG, "null array or no SMs");
+        XG_REQUIRE(M > 0 && N > 0 && K > 0 && M % 128 == 0 && N % 128 == 0 && K % 64 == 0,
+                   XAMG_ERR_INVALID_ARG,
+                   "gemm: M and N must be multiples of 128, K a positive multiple of 64");
+        // index [width 64, 128, 256][split 1, 2, 4, 8]
+        auto given = [&](int bn, int split) {
+            return cluster_ctas[(bn / 128) * 4 + (split == 8 ? 3 : split / 2)];
+        };
+        const ops::mm::Shape sh =
+            cluster_ctas ? ops::mm::shape_for(M, N, K, sms, may_split != 0, transposed != 0, given)
+                         : ops::mm::gemm_shape(M, N, K, may_split != 0, transposed != 0);
+        shape[0] = sh.bn;
+        shape[1] = sh.split;
+        shape[2] = sh.stages;
+    });
+}
+
 static std::vector<std::unique_ptr<Mlp>> g_mlps;
 
 int XAMG_b200_mlp_create(uint32_t n_in, uint32_t n_hidden, uint32_t n_out, uint64_t seed,

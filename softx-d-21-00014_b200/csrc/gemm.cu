@@ -27,13 +27,13 @@
 #include <cuda_bf16.h>
 
 #include "device.h"
+#include "gemm_shape.h"
 #include "ops.h"
 
 namespace xg {
 namespace ops {
 namespace mm {
 
-constexpr int BM = 128, BK = 64;
 constexpr int MAX_STAGES = 8;
 constexpr int THREADS = 320;
 constexpr uint32_t BOX = 64 * BK * 2;  // one 64 x 64 TMA box of a transposed operand
@@ -429,18 +429,6 @@ __global__ void __launch_bounds__(THREADS, 2)
 
 namespace {
 
-// Tile width, K split and stages. What bounds a tile is the operands' way from
-// L2: a k-block of a 128 x BN tile is (128 + BN) x 128 bytes, about 48 bytes a
-// clock into each of 148 SMs (T_KB us a 128 x 128 block), after T_FIXED us of
-// start and epilogue; a split costs T_SPLIT for the exchange. One CTA an SM
-// with 192 KB of operands in flight, or two of 96 KB (128 x 128 tiles), whose
-// epilogues then overlap the other's main loop. The cheapest shape of the waves
-// this makes.
-struct Shape {
-    int bn, split, stages;
-};
-constexpr double T_KB = 0.35, T_FIXED = 4.0, T_SPLIT = 1.5;
-
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     if (!fn) {
@@ -470,9 +458,6 @@ CUtensorMap make_map(const void *ptr, uint64_t rows, uint64_t cols, uint32_t box
     return m;
 }
 
-// One CTA an SM: 192 KB of operands in flight.
-constexpr int stages_for(int bn) { return bn == 256 ? 4 : bn == 128 ? 6 : 8; }
-
 template <int BN, int MODE>
 void allow_smem() {
     static bool attr = false;  // one flag per instantiation
@@ -487,7 +472,7 @@ void allow_smem() {
 // CTAs of clusters of `split` that the GPU holds at once (a cluster lies within
 // one GPC, so this is fewer than one an SM).
 template <int BN>
-int query_cluster_ctas(int split, int sms) {
+int query_cluster_ctas(int split) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)split * 64);
     cfg.blockDim = dim3(THREADS);
@@ -502,46 +487,18 @@ int query_cluster_ctas(int split, int sms) {
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16<BN, F32>, &cfg) != cudaSuccess || n < 1) {
         cudaGetLastError();
-        n = std::max(1, sms / split / 2);
+        n = std::max(1, ctx().sms / split / 2);
     }
     return n * split;
 }
-int cluster_ctas(int bn, int split, int sms) {
+int cluster_ctas(int bn, int split) {
     static int known[3][9] = {};
     int &n = known[bn == 256 ? 2 : bn == 128 ? 1 : 0][split];
     if (!n)
-        n = bn == 256   ? query_cluster_ctas<256>(split, sms)
-            : bn == 128 ? query_cluster_ctas<128>(split, sms)
-                        : query_cluster_ctas<64>(split, sms);
+        n = bn == 256   ? query_cluster_ctas<256>(split)
+            : bn == 128 ? query_cluster_ctas<128>(split)
+                        : query_cluster_ctas<64>(split);
     return n;
-}
-
-Shape shape_for(uint64_t M, uint64_t N, uint64_t K, int sms, bool may_split) {
-    const uint64_t KB = K / BK;
-    Shape best{128, 1, 6};
-    double cost = 1e300;
-    auto consider = [&](int bn, int split, int stages, double c) {
-        if (c < cost) {
-            cost = c;
-            best = Shape{bn, split, stages};
-        }
-    };
-    auto waves = [&](uint64_t ctas, int slots) { return (double)((ctas + slots - 1) / slots); };
-    for (int bn : {256, 128, 64}) {
-        if (N % (uint64_t)bn) continue;
-        const double kb = T_KB * (128 + bn) / 256.0;
-        for (int split : {1, 2, 4, 8}) {
-            if (split > 1 && (!may_split || KB < 4ull * split)) break;
-            const uint64_t ctas = (M / BM) * (N / bn) * split;
-            consider(bn, split, stages_for(bn),
-                     waves(ctas, split > 1 ? cluster_ctas(bn, split, sms) : sms) *
-                         ((double)((KB + split - 1) / split) * kb + T_FIXED +
-                                         (split > 1 ? T_SPLIT : 0.0)));
-        }
-        if (bn == 128)
-            consider(bn, 1, 3, waves((M / BM) * (N / bn), 2 * sms) * (2 * (double)KB * kb + T_FIXED));
-    }
-    return best;
 }
 
 template <int BN, int MODE>
@@ -588,7 +545,7 @@ uint64_t run(uint64_t M, uint64_t N, uint64_t K, const void *A, bool a_mn, const
     XG_REQUIRE(((uintptr_t)A | (uintptr_t)B | (uintptr_t)ep.C) % 16 == 0, XAMG_ERR_INVALID_ARG,
                "gemm: A, B and C must be 16-byte aligned");
     XG_REQUIRE(M / BM <= 65535, XAMG_ERR_INVALID_ARG, "gemm: M too large");
-    const Shape sh = shape_for(M, N, K, ctx().sms, may_split);
+    const Shape sh = shape_for(M, N, K, ctx().sms, may_split, a_mn && b_mn, cluster_ctas);
     const CUtensorMap ta = a_mn ? make_map(A, K, M, BK) : make_map(A, M, K, BM);
     const CUtensorMap tb = b_mn ? make_map(B, K, N, BK) : make_map(B, N, K, (uint32_t)sh.bn);
     if (sh.bn == 256)
@@ -601,6 +558,10 @@ uint64_t run(uint64_t M, uint64_t N, uint64_t K, const void *A, bool a_mn, const
 }
 
 }  // namespace
+
+Shape gemm_shape(uint64_t M, uint64_t N, uint64_t K, bool may_split, bool mn) {
+    return shape_for(M, N, K, ctx().sms, may_split, mn, cluster_ctas);
+}
 
 void gemm_bf16(uint64_t M, uint64_t N, uint64_t K, const void *A, const void *B, void *C,
                uint64_t ldc, int mode, const float *bias, const void *aux, uint64_t ld_aux,

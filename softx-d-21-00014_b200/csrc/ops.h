@@ -5,6 +5,7 @@
 #pragma once
 
 #include "device.h"
+#include "gemm_shape.h"
 
 namespace xg {
 namespace ops {
@@ -93,6 +94,8 @@ namespace mm {
 void gemm_bf16(uint64_t M, uint64_t N, uint64_t K, const void *A, const void *B, void *C,
                uint64_t ldc, int mode, const float *bias, const void *aux, uint64_t ld_aux,
                cudaStream_t s, bool a_mn = false, bool b_mn = false, bool may_split = true);
+// the shape that such a GEMM takes on this GPU (gemm_shape.h); mn: a_mn and b_mn
+Shape gemm_shape(uint64_t M, uint64_t N, uint64_t K, bool may_split, bool mn);
 // a_mn / b_mn: A is stored transposed as [K][M], B as [K][N]. may_split: the
 // sum over K may be split between CTAs (another rounding of the same sums).
 // The last layer of a training pass: d = A B^T + bias - T, dY[M][N] = scale d

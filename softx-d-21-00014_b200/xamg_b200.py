@@ -63,6 +63,7 @@ EXT_SYMBOLS = [
     "XAMG_b200_mlp_gradients", "XAMG_b200_mlp_params", "XAMG_b200_solver_solve_batch",
     "XAMG_b200_solver_level_tuned", "XAMG_b200_stencil_layout", "XAMG_b200_solver_level_stencil",
     "XAMG_b200_solver_level_xstaged", "XAMG_b200_solver_level_hsgs",
+    "XAMG_b200_gemm_shape",
 ]
 
 
@@ -190,6 +191,7 @@ def lib():
         "XAMG_b200_solver_hierarchy_save": (C.c_int, [C.c_size_t, C.c_char_p]),
         "XAMG_b200_gemm_bf16": (C.c_int, [u64, u64, u64, vp, vp, vp, u64, C.c_int, vp, vp, u64,
                                           vp]),
+        "XAMG_b200_gemm_shape": (C.c_int, [u64, u64, u64, C.c_int, C.c_int, C.c_int, vp, vp]),
         "XAMG_b200_mlp_create": (C.c_int, [C.c_uint32, C.c_uint32, C.c_uint32, u64,
                                            C.POINTER(C.c_size_t)]),
         "XAMG_b200_mlp_destroy": (C.c_int, [C.c_size_t]),
@@ -282,6 +284,15 @@ def stencil_layout(row, col):
     call("XAMG_b200_stencil_layout", len(row) - 1, _ptr(row), _ptr(col), C.byref(pat),
          C.byref(S), C.byref(S2), C.byref(df))
     return pat.value, S.value, S2.value, df.value
+
+
+def gemm_shape(M, N, K, may_split=True, sms=0, cluster_ctas=None, transposed=False):
+    """(tile width, K split, stages) of a GEMM; cluster_ctas: 12 values, see the header."""
+    out = np.zeros(3, np.int32)
+    c = None if cluster_ctas is None else np.ascontiguousarray(cluster_ctas, np.int32)
+    call("XAMG_b200_gemm_shape", M, N, K, int(may_split), int(transposed), sms, None if c is None else _ptr(c),
+         _ptr(out))
+    return tuple(int(v) for v in out)
 
 
 def generate_cube(nx, ny, nz):
