@@ -470,7 +470,8 @@ void allow_smem() {
 }
 
 // CTAs of clusters of `split` that the GPU holds at once (a cluster lies within
-// one GPC, so this is fewer than one an SM).
+// one GPC, so this is fewer than one an SM); 0 where it holds none or the query
+// fails.
 template <int BN>
 int query_cluster_ctas(int split) {
     cudaLaunchConfig_t cfg = {};
@@ -485,20 +486,20 @@ int query_cluster_ctas(int split) {
     cfg.numAttrs = 1;
     allow_smem<BN, F32>();
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16<BN, F32>, &cfg) != cudaSuccess || n < 1) {
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_bf16<BN, F32>, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        n = std::max(1, ctx().sms / split / 2);
+        n = 0;
     }
     return n * split;
 }
 int cluster_ctas(int bn, int split) {
-    static int known[3][9] = {};
+    static int known[3][9] = {};  // 1 + the CTAs; 0: not asked yet
     int &n = known[bn == 256 ? 2 : bn == 128 ? 1 : 0][split];
     if (!n)
-        n = bn == 256   ? query_cluster_ctas<256>(split)
-            : bn == 128 ? query_cluster_ctas<128>(split)
-                        : query_cluster_ctas<64>(split);
-    return n;
+        n = 1 + (bn == 256   ? query_cluster_ctas<256>(split)
+                 : bn == 128 ? query_cluster_ctas<128>(split)
+                             : query_cluster_ctas<64>(split));
+    return n - 1;
 }
 
 template <int BN, int MODE>

@@ -35,7 +35,8 @@ constexpr double t_kb_mn(int bn) { return bn == 256 ? 0.08 : bn == 128 ? 0.03 : 
 constexpr int stages_for(int bn) { return bn == 256 ? 4 : bn == 128 ? 6 : 8; }
 
 // cluster_ctas(bn, split): CTAs of clusters of `split` that the GPU holds at
-// once. mn: both operands are transposed.
+// once; 0 where it holds none, and then no shape has that split. mn: both operands
+// are transposed.
 template <class Ctas>
 Shape shape_for(uint64_t M, uint64_t N, uint64_t K, int sms, bool may_split, bool mn,
                 const Ctas &cluster_ctas) {
@@ -55,6 +56,7 @@ Shape shape_for(uint64_t M, uint64_t N, uint64_t K, int sms, bool may_split, boo
         for (int split : {1, 2, 4, 8}) {
             if (split > 1 && (!may_split || KB < 4ull * split)) break;
             const int slots = split > 1 ? cluster_ctas(bn, split) : sms;
+            if (slots < split) continue;
             const uint64_t ctas = (M / BM) * (N / bn) * split;
             consider(bn, split, stages_for(bn),
                      waves(ctas, slots) * ((double)((KB + split - 1) / split) * kb + t_tile(bn) +

@@ -10,6 +10,29 @@ SHAPES = [(128, 256, 5248), (128, 1024, 5248), (128, 5248, 1024), (512, 5248, 10
           (4096, 1024, 5248), (2176, 1408, 704), (128, 128, 64), (65536, 128, 1024)]
 
 
+def waves(shape, M, N, ctas, sms):
+    bn, split, stages = shape
+    slots = ctas[{64: 0, 128: 1, 256: 2}[bn], {1: 0, 2: 1, 4: 2, 8: 3}[split]] if split > 1 \
+        else sms * (2 if stages == 3 else 1)
+    return -(-(M // 128) * (N // bn) * split // slots)
+
+
+@pytest.mark.parametrize("none", [(), (2,), (8,), (2, 4), (2, 4, 8)])
+def test_no_split_the_gpu_cannot_hold(xamg, none):
+    """A cluster size of which the GPU holds none is never chosen."""
+    ctas = CTAS.copy()
+    for s in none:
+        ctas[:, {2: 1, 4: 2, 8: 3}[s]] = 0
+    splits = set()
+    for M, N, K in SHAPES:
+        bn, split, stages = xamg.gemm_shape(M, N, K, True, 148, ctas)
+        assert N % bn == 0 and split not in none and K // 64 >= (4 * split if split > 1 else 1)
+        assert 3 <= stages <= 8 and stages * (128 + bn) * 128 <= 192 * 1024
+        assert waves((bn, split, stages), M, N, ctas, 148) >= 1
+        splits.add(split)
+    assert (max(splits) > 1) == (len(none) < 3)
+
+
 def test_training_products_never_split(xamg):
     for M, N, K in SHAPES:
         assert xamg.gemm_shape(M, N, K, False, 148, CTAS)[1] == 1
