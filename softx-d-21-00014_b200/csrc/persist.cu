@@ -18,7 +18,7 @@ template <int NV, typename I>
 static bool fits_nv(uint64_t n, int share) {
     const int B = k::canon_blocks(n, NV);
     if ((uint64_t)B * NV * 8 > (uint64_t)k::BMAX * 32 * 4) return false;
-    const int res = resident_blocks(k::k_pbicgstab_persist<NV, I>, k::CT, 0);
+    const int res = occupancy(k::k_pbicgstab_persist<NV, I>, k::CT, 0);
     return (uint64_t)res * (uint64_t)ctx().sms >= (uint64_t)grid_of(B, share);
 }
 
@@ -51,8 +51,7 @@ static uint32_t reg_blocks(const DCsr &A, int sweeps, int share, uint32_t &smem,
                                      (int)REG_SMEM_MAX));
         big_smem = true;
     }
-    const int res = resident_blocks(kern, k::CT, smem);
-    return res >= 1 ? (uint32_t)ntiles : 0;
+    return occupancy(kern, k::CT, smem) >= 1 ? (uint32_t)ntiles : 0;
 }
 
 size_t pbicgstab_exchange_bytes(const DCsr &A, int nv, int sweeps, int share) {

@@ -82,18 +82,23 @@ static uint32_t stage_buffer_bytes(uint32_t cap) {
 }
 
 // Resident blocks per SM of a kernel for a dynamic shared-memory size
-// (remembered per kernel and size).
+// (remembered per kernel and size); 0 where it does not fit an SM.
 template <class Kern>
-static int resident_blocks(Kern kern, int threads, size_t smem) {
+static int occupancy(Kern kern, int threads, size_t smem) {
     static std::map<std::pair<const void *, size_t>, int> cache;
     const auto key = std::make_pair((const void *)kern, smem);
     auto it = cache.find(key);
     if (it == cache.end()) {
         int nb = 0;
         XG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, threads, smem));
-        it = cache.emplace(key, std::max(nb, 1)).first;
+        it = cache.emplace(key, nb).first;
     }
     return it->second;
+}
+// The same for sizing a grid: at least one.
+template <class Kern>
+static int resident_blocks(Kern kern, int threads, size_t smem) {
+    return std::max(occupancy(kern, threads, smem), 1);
 }
 
 // Grid: as many blocks as fit the GPU at once (one wave). With dot products
