@@ -40,6 +40,7 @@ struct DevBuf {
             cudaError_t e = cudaMalloc(&p, b);
             if (e != cudaSuccess) {
                 p = nullptr;
+                cudaGetLastError();  // not for the next launch to find
                 throw Error(XAMG_ERR_ALLOC, std::string("cudaMalloc(") + std::to_string(b) +
                                                 " bytes): " + cudaGetErrorString(e));
             }

@@ -168,7 +168,7 @@ void Mlp::ensure(uint32_t batch) {
     XG_REQUIRE(batch > 0 && batch % 128 == 0, XAMG_ERR_INVALID_ARG,
                "mlp: the batch must be a positive multiple of 128");
     if (batch <= cap) return;
-    cap = batch;
+    cap = 0;  // until every buffer is there: an allocation may throw
     const uint64_t B = batch;
     X.alloc(B * n_in * 2);
     H1.alloc(B * h * 2);
@@ -182,6 +182,7 @@ void Mlp::ensure(uint32_t batch) {
     sse_host = nullptr;
     XG_CUDA(cudaMallocHost((void **)&sse_host, parts * sizeof(double)));
     if (!sse_ready) XG_CUDA(cudaEventCreateWithFlags(&sse_ready, cudaEventDisableTiming));
+    cap = batch;
 }
 
 Mlp::~Mlp() {

@@ -100,3 +100,23 @@ def test_training_reduces_the_loss(gpu):
     for _ in range(300):
         last = m.train_step(Xd.data_ptr(), Td.data_ptr(), B, 1e-3)
     assert last < first / 10, (first, last)
+
+
+def test_a_batch_that_does_not_fit_leaves_the_network_usable(gpu):
+    """A batch whose activations exceed the device's memory (274 GB for the inputs
+    alone) is refused every time it is asked for, not only the first, and the
+    network then works as before."""
+    import torch
+    n_in, h, n_out, B = 128, 128, 128, 128
+    X = torch.randn(B, n_in, device="cuda")
+    T = torch.randn(B, n_out, device="cuda")
+    Y = torch.empty(B, n_out, device="cuda")
+    torch.cuda.synchronize()
+    m = gpu.Mlp(n_in, h, n_out, seed=1)
+    g0, l0 = m.gradients(X.data_ptr(), T.data_ptr(), B)
+    for _ in range(2):
+        with pytest.raises(gpu.XamgError) as e:
+            m.predict(X.data_ptr(), Y.data_ptr(), 1 << 30)
+        assert e.value.code == -9
+    g1, l1 = m.gradients(X.data_ptr(), T.data_ptr(), B)
+    assert l0 == l1 and g0.tobytes() == g1.tobytes()
