@@ -1095,9 +1095,10 @@ int XAMG_b200_mlp_train_step(size_t id, uint32_t batch, const float *X, const fl
                              double *loss) {
     return guarded([&] {
         XG_REQUIRE(X && T, XAMG_ERR_INVALID_ARG, "null argument");
-        const double l = get(g_mlps, id, "mlp").train_step(batch, X, T, lr);
-        if (loss) *loss = l;
-        ctx().check_flags();
+        Mlp &m = get(g_mlps, id, "mlp");
+        m.train_step(batch, X, T, lr);
+        ctx().check_flags();  // waits for the step
+        if (loss) *loss = m.loss();
     });
 }
 
@@ -1106,10 +1107,10 @@ int XAMG_b200_mlp_gradients(size_t id, uint32_t batch, const float *X, const flo
     return guarded([&] {
         XG_REQUIRE(X && T && grads, XAMG_ERR_INVALID_ARG, "null argument");
         Mlp &m = get(g_mlps, id, "mlp");
-        const double l = m.gradients(batch, X, T);
+        m.backward(batch, X, T);
         m.copy_params(grads, false, true);
-        if (loss) *loss = l;
         ctx().check_flags();
+        if (loss) *loss = m.loss();
     });
 }
 

@@ -181,7 +181,6 @@ void Mlp::ensure(uint32_t batch) {
     if (sse_host) XG_CUDA(cudaFreeHost(sse_host));
     sse_host = nullptr;
     XG_CUDA(cudaMallocHost((void **)&sse_host, parts * sizeof(double)));
-    if (!sse_ready) XG_CUDA(cudaEventCreateWithFlags(&sse_ready, cudaEventDisableTiming));
     cap = batch;
 }
 
@@ -190,7 +189,6 @@ Mlp::~Mlp() {
     for (cudaStream_t c : copy_streams)
         if (c) cudaStreamDestroy(c);
     if (sse_host) cudaFreeHost(sse_host);
-    if (sse_ready) cudaEventDestroy(sse_ready);
 }
 
 // The first two layers, activations kept in BF16.
@@ -226,8 +224,8 @@ void Mlp::backward(uint32_t batch, const float *Xf, const float *T) {
     // dH2 = dY W3 masked by H2 > 0
     sse_n = ops::mm::gemm_mse_grad(B, n_out, h, H2.p, layer[2].wt_bf.p, dY.p,
                                    layer[2].b.as<float>(), T, scale, sse.as<double>(), S());
+    loss_n = B * n_out;
     XG_CUDA(cudaMemcpyAsync(sse_host, sse.p, sse_n * sizeof(double), cudaMemcpyDeviceToHost, S()));
-    XG_CUDA(cudaEventRecord(sse_ready, S()));
     gemm_bf16(n_out, h, B, dY.p, H2.p, layer[2].gw.p, h, 0, nullptr, nullptr, 0, S(), true, true,
               false);
     gemm_bf16(B, h, n_out, dY.p, layer[2].wt_bf.p, dH2.p, h, 3, nullptr, H2.p, h, S(), false, true,
@@ -250,21 +248,13 @@ void Mlp::backward(uint32_t batch, const float *Xf, const float *T) {
     XG_CUDA(cudaGetLastError());
 }
 
-// The loss of the last backward pass (waits for its partial sums only).
-double Mlp::loss(uint32_t batch) {
-    XG_CUDA(cudaEventSynchronize(sse_ready));
+double Mlp::loss() const {
     double s = 0;
     for (uint64_t i = 0; i < sse_n; ++i) s += sse_host[i];
-    return s / (double)((uint64_t)batch * n_out);
+    return s / (double)loss_n;
 }
 
-double Mlp::gradients(uint32_t batch, const float *Xf, const float *T) {
-    backward(batch, Xf, T);
-    XG_CUDA(cudaStreamSynchronize(S()));
-    return loss(batch);
-}
-
-double Mlp::train_step(uint32_t batch, const float *Xf, const float *T, float lr) {
+void Mlp::train_step(uint32_t batch, const float *Xf, const float *T, float lr) {
     backward(batch, Xf, T);
     ++step;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
@@ -283,7 +273,6 @@ double Mlp::train_step(uint32_t batch, const float *Xf, const float *T, float lr
     k_adam<<<grid_for(most), 256, 0, S()>>>(a, lr, b1, b2, eps, c1, c2);
     ++g_kernel_launches;
     XG_CUDA(cudaGetLastError());
-    return loss(batch);
 }
 
 // Device values to the caller's pageable memory. One cudaMemcpy moves 5 GB/s

@@ -22,7 +22,7 @@ struct Mlp {
     DevBuf sse;                  // the loss's partial sums (one per CTA of the last layer)
     double *sse_host = nullptr;  // their pinned copy
     uint64_t sse_n = 0;
-    cudaEvent_t sse_ready = nullptr;
+    uint64_t loss_n = 0;  // outputs the loss is a mean over
     // parameter read-back: pinned buffers and streams of its copying threads
     static constexpr int COPIERS = 4;
     char *bounce = nullptr;
@@ -36,11 +36,13 @@ struct Mlp {
     void init(uint32_t n_in, uint32_t n_hidden, uint32_t n_out, uint64_t seed);
     // Y = MLP(X) for `batch` rows of FP32 X [batch][n_in] into FP32 Y
     void forward(uint32_t batch, const float *X, float *Y);
-    // gradients of the mean squared error against T at the current weights;
-    // returns the loss
-    double gradients(uint32_t batch, const float *X, const float *T);
-    // one Adam step; returns the loss before the step
-    double train_step(uint32_t batch, const float *X, const float *T, float lr);
+    // gradients of the mean squared error against T at the current weights
+    void backward(uint32_t batch, const float *X, const float *T);
+    // one Adam step
+    void train_step(uint32_t batch, const float *X, const float *T, float lr);
+    // the loss of the last backward pass, before its step; once the stream has
+    // been waited for
+    double loss() const;
     uint64_t param_count() const;
     void copy_params(float *host, bool set, bool grads);
 
@@ -49,8 +51,6 @@ struct Mlp {
     void ensure(uint32_t batch);
     void refresh_bf16();
     void hidden(uint32_t batch, const float *X, bool split);
-    void backward(uint32_t batch, const float *X, const float *T);
-    double loss(uint32_t batch);
     static cudaStream_t S() { return ctx().stream; }
 };
 
