@@ -92,3 +92,19 @@ def test_gemm_unaligned_bias_and_padded_rows(gpu):
     got = C.cpu().double().numpy()
     assert np.all(np.abs(got[:, :N] - ref) <= bound)
     assert np.all(got[:, N:] == 7.0)
+
+
+@pytest.mark.parametrize("M,N,K,mode,shape", [
+    (128, 128, 64, 0, (64, 1, 8)), (512, 1024, 704, 2, (64, 1, 8)),
+    (384, 384, 1024, 3, (64, 4, 8)), (128, 256, 2368, 1, (64, 8, 8)),
+    (1280, 1024, 704, 0, (128, 1, 6)), (1280, 1024, 704, 3, (128, 1, 6)),
+    (1280, 640, 2368, 2, (128, 2, 6)), (256, 1152, 2368, 0, (128, 4, 6)),
+    (2176, 1408, 704, 0, (128, 1, 3)), (2176, 2304, 704, 2, (128, 1, 3)),
+    (2176, 1408, 704, 3, (128, 1, 3)), (1280, 2304, 1088, 0, (256, 1, 4)),
+    (1280, 2304, 1088, 3, (256, 1, 4)), (1280, 1024, 2368, 2, (256, 2, 4))])
+def test_gemm_shapes(gpu, M, N, K, mode, shape):
+    """Every tile width with and without a K split, one CTA an SM and two, fewer
+    tiles than SMs and more, k-blocks that the split does not divide."""
+    assert gpu.gemm_shape(M, N, K) == shape
+    got, ref, bound = run(gpu, M, N, K, mode, seed=M + K)
+    assert np.all(np.abs(got - ref) <= bound), np.abs(got - ref).max()

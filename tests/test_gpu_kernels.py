@@ -210,6 +210,61 @@ def test_spmv_dot_fused(gpu, oracle, nv):
         oracle.set_reduction(0)
 
 
+def shifted(a, d):
+    """a on the device, d elements behind a 16-byte boundary: (buffer, address)."""
+    buf = torch_dev(np.concatenate([np.full(d, 9.0, a.dtype), a]))
+    return buf, buf.data_ptr() + d * a.itemsize
+
+
+@pytest.mark.parametrize("nv", [2, 4, 8])
+@pytest.mark.parametrize("dx,dv,dz", [(1, 0, 0), (2, 0, 0), (4, 0, 0), (0, 1, 0), (0, 0, 1),
+                                      (2, 2, 2)])
+def test_spmv_dot_unaligned_vectors(gpu, oracle, nv, dx, dv, dz):
+    """A caller's x on 16 bytes but not 32 (two right-hand sides a thread), and x, v
+    or z on 8 (one): the same product and the same order of the sums."""
+    rng = np.random.default_rng(nv + dx)
+    n = 700
+    row, col, val = random_csr(n, n, rng)
+    x, z = rng.standard_normal(n * nv), rng.standard_normal(n * nv)
+    A, keep = dev_csr(gpu, row, col, val, n, 2, False)
+    (xb, xp), (vb, vp), (zb, zp) = shifted(x, dx), shifted(np.zeros(n * nv), dv), shifted(z, dz)
+    dot = np.zeros(nv)
+    gpu.call("XAMG_b200_spmv_dot", C.byref(A), xp, vp, zp, dot.ctypes.data_as(C.c_void_p), nv,
+             None)
+    v = oracle.csr_ax_y(row, col, val, x, nv, ncols=n)
+    got = vb.cpu().numpy()
+    assert got[dv:].tobytes() == v.tobytes() and np.all(got[:dv] == 9.0)
+    oracle.set_reduction(1)
+    try:
+        assert dot.tobytes() == oracle.dot(v, z, nv).tobytes()
+    finally:
+        oracle.set_reduction(0)
+
+
+@pytest.mark.parametrize("nv", [2, 4, 8])
+@pytest.mark.parametrize("which", range(4))
+def test_group4_unaligned_vectors(gpu, oracle, nv, which):
+    """Group 4 with one of s, t, r0 and r on 8 bytes."""
+    rng = np.random.default_rng(nv)
+    n = 5000
+    s, t, r0, r = (rng.standard_normal(n * nv) for _ in range(4))
+    om = rng.standard_normal(nv)
+    bufs = [shifted(a, int(q == which)) for q, a in enumerate((s, t, r0, r))]
+    rho = np.zeros(nv)
+    gpu.call("XAMG_b200_group4", n, nv, *[p for _, p in bufs], om.ctypes.data_as(C.c_void_p),
+             rho.ctypes.data_as(C.c_void_p), None)
+    o_r, o_rho = np.zeros(n * nv), np.zeros(nv)
+    oracle.set_reduction(1)
+    try:
+        oracle.lib().or_group4(n, nv, s, t, r0, o_r, om, o_rho)
+    finally:
+        oracle.set_reduction(0)
+    got = bufs[3][0].cpu().numpy()
+    d = int(which == 3)
+    assert got[d:].tobytes() == o_r.tobytes() and np.all(got[:d] == 9.0)
+    assert rho.tobytes() == o_rho.tobytes()
+
+
 def test_kernels_are_sm100_machine_code(gpu):
     """The CUDA runtime reports the library's kernels as sm_100 machine code."""
     import ctypes as C

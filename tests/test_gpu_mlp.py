@@ -47,15 +47,22 @@ def test_gradients_against_oracle(gpu, n_in, h, n_out, B):
         assert np.abs(gb - rb).max() <= 1e-2 * np.abs(rb).max() + 1e-12
 
 
-@pytest.mark.parametrize("n_in,h,n_out,B", [(640, 384, 1152, 384), (256, 1024, 128, 640)])
-def test_gradients_of_several_tiles(gpu, n_in, h, n_out, B):
-    """Several tiles and K splits in every product, transposed operands included.
+@pytest.mark.parametrize("n_in,h,n_out,B,widths",
+                         [(640, 384, 1152, 384, {64}), (256, 1024, 128, 640, {64}),
+                          (1408, 1280, 2176, 1280, {128})])
+def test_gradients_of_several_tiles(gpu, n_in, h, n_out, B, widths):
+    """Several tiles in every product, transposed operands included, in tiles of 64
+    columns and of 128 (one CTA an SM and two); training products never split K.
     With B x h activations a pre-activation within the FP32 accumulation's error
     of zero can fall on the other side of the ReLU than in the oracle: that
     moves one sample's share of one row of a weight gradient, about
     1 / sqrt(B h) of the block's norm (0.3 % here), so blocks are compared in
     the 2-norm, 1 % allowing some ten of them."""
     import torch
+    shapes = [gpu.gemm_shape(*mnk, False, transposed=True)
+              for mnk in ((n_out, h, B), (h, h, B), (h, n_in, B))]
+    assert {s[0] for s in shapes} == widths and {s[1] for s in shapes} == {1}
+    assert widths == {64} or {s[2] for s in shapes} == {3, 6}
     m = gpu.Mlp(n_in, h, n_out, seed=3)
     p = m.params()
     rng = np.random.default_rng(4)
