@@ -144,7 +144,10 @@ int XAMG_b200_solver_level_info(size_t sid, int level, int which, uint64_t *nrow
 
 /* The SpMV launch shapes the autotuner (parameter gpu_spmv_tune, default 1)
  * picked for level matrix `which` (no counterpart): 24 codes, index
- * [value type is float][x type is float][log2 nv]; 0 = not tuned (yet), else
+ * [value type is float][x type is float][log2 nv]. The plain products (y = A x,
+ * y += A x, prolongation) and the smoothers' steps and residuals have a shape
+ * each; the code is that of the plain products where they have been measured.
+ * 0 = not tuned (yet), else
  * 1 + 9 * (right-hand sides a thread: 0 the default of 2 for double and 4 for
  * float x, 1 the other one, 2 eight for float x at nv >= 8) + 3 * (staging: 0 one
  * buffer, 1 two, 2 none) +

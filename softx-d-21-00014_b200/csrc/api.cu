@@ -927,7 +927,11 @@ int XAMG_b200_solver_level_tuned(size_t sid, int level, int which, uint8_t *code
     return guarded([&] {
         XG_REQUIRE(codes, XAMG_ERR_INVALID_ARG, "null array");
         const DCsr &d = level_matrix(sid, level, which);
-        std::memcpy(codes, &d.tuned[0][0][0], 24);
+        for (int i = 0; i < 24; ++i) {
+            codes[i] = 0;
+            for (int e = 0; e < k::TK_COUNT && !codes[i]; ++e)
+                codes[i] = (&d.tuned[e][0][0][0])[i];
+        }
     });
 }
 

@@ -145,14 +145,14 @@ struct DCsr {
     // (index log2 nv); 0 = not known yet
     uint32_t tile_max[6] = {0, 0, 0, 0, 0, 0};
     // SpMV autotuning (library-owned matrices, gpu_spmv_tune): the launch
-    // shape measured fastest for the SpMVs without dot products, per
+    // shape measured fastest for the SpMVs without dot products, per [kind, k::TuneKind]
     // [value type is float][x type is float][log2 nv]: 0 = not tuned yet,
     // else 1 + 9 * (right-hand sides a thread: 0 default, 1 alternative, 2
     // eight) + 3 * (staging: 0 one buffer, 1 two, 2 none) + (tile run: 0 one,
     // 1 four, 2 sixteen), or 28: the warp-per-row kernel (k_spmv_wide), or
     // 29 + 3 * (right-hand sides a thread) + (staging): the plane walk
     bool tune_on = false;
-    mutable uint8_t tuned[2][2][6] = {};
+    mutable uint8_t tuned[k::TK_COUNT][2][2][6] = {};
     // Plane walk (square matrices with long-range neighbours): walk_rows is
     // the distance, in rows, from a middle row to the centre of its farthest
     // neighbour cluster (the next grid plane of a structured grid; 0: none).
@@ -172,9 +172,9 @@ struct DCsr {
     bool st_diag_first = false;  // rows store their diagonal first
     DevBuf st_val, st_mask;
     // with tuning on: the kernel measured fastest for the SpMVs without dot
-    // products, per [value type is float][log2 nv]: 0 = not tuned yet, 1 the
+    // products, per [kind][value type is float][log2 nv]: 0 = not tuned yet, 1 the
     // stencil kernel with 64 registers a thread, 2 with 128, 3 the CSR kernel
-    mutable uint8_t st_choice[2][6] = {};
+    mutable uint8_t st_choice[k::TK_COUNT][2][6] = {};
     uint8_t st_force = 0;     // gpu_spmv_tune = 2: always the 128-register form
     bool wide_force = false;  // gpu_spmv_tune = 3: the warp-per-row kernel where allowed
     bool xs_force = false;    // gpu_spmv_tune = 4: the x-staged kernel where built

@@ -863,6 +863,13 @@ struct NoFin {
     __device__ void operator()(int, const T *) const {}
 };
 
+// The epilogues of SpMVs without dot products, as the autotuner tells them apart:
+// plain products, which read at most y beside the sum, and the smoothers' steps and
+// residuals with their vectors. Each kind has a launch shape of its own in the
+// matrix (DCsr::tuned, DCsr::st_choice), so that a product that somebody asks for
+// does not decide the smoother's.
+enum TuneKind : int { TK_PLAIN = 0, TK_SMOOTH, TK_COUNT };
+
 // What every SpMV epilogue shares: a row sum that starts from zero, and the
 // one-right-hand-side forms written with the vector ones. (redirect, where there
 // are no dot products: the outputs go to scratch vectors a and b; the autotuner
@@ -890,6 +897,7 @@ struct EpiBase {
 // y = A x  (csr_matvec.inl:213-231)
 template <typename F, int NV>
 struct EStore : EpiBase<EStore<F, NV>, F>, NoFin {
+    static constexpr int KIND = TK_PLAIN;
     F *y;
     __host__ __device__ explicit EStore(F *y_) : y(y_) {}
     bool aligned() const { return aligned16(y); }
@@ -911,6 +919,7 @@ struct EStore : EpiBase<EStore<F, NV>, F>, NoFin {
 // y += A x  (csr_matvec.inl:106-120: accumulate directly into y)
 template <typename F, int NV>
 struct EAxpy : NoFin {
+    static constexpr int KIND = TK_PLAIN;
     static constexpr size_t SCRATCH_A = sizeof(F), SCRATCH_B = 0;
     F *y;
     __host__ __device__ explicit EAxpy(F *y_) : y(y_) {}
@@ -944,6 +953,7 @@ struct EAxpy : NoFin {
 // optionally with (r, r) (vector_norm, blas.inl:537-555).
 template <typename F, int NV, bool NORM>
 struct EResid : EpiBase<EResid<F, NV, NORM>, F> {
+    static constexpr int KIND = TK_SMOOTH;
     F *r;
     const F *b;
     double *out;  // NORM: sums land here (nv values)
@@ -1099,6 +1109,7 @@ struct EDot3 : EpiBase<EDot3<NV>, double> {
 // x_out = x_in + relax*d*(b - A x_in)
 template <typename F, int NV>
 struct EJacobi : EpiBase<EJacobi<F, NV>, F>, NoFin {
+    static constexpr int KIND = TK_SMOOTH;
     F *xout;
     const F *xin, *b, *d;
     F relax;
@@ -1131,6 +1142,7 @@ struct EJacobi : EpiBase<EJacobi<F, NV>, F>, NoFin {
 // SpMV). x_zero: r = 1*b without the SpMV (used by k_rows through elem()).
 template <typename F, int NV>
 struct ECheby0 : EpiBase<ECheby0<F, NV>, F>, NoFin {
+    static constexpr int KIND = TK_SMOOTH;
     static constexpr size_t SCRATCH_B = sizeof(F);
     F *rs, *t1s;
     const F *b, *isd;
@@ -1227,6 +1239,7 @@ struct ECheby0From64 : NoFin {
 // (more steps) or x = 1*(t1*isd) + 1*x (last step; x_zero: x = 1*(t1*isd)).
 template <typename F, int NV>
 struct ECheby1 : EpiBase<ECheby1<F, NV>, F>, NoFin {
+    static constexpr int KIND = TK_SMOOTH;
     F *out;  // next t1s, or x on the last step
     const F *rs, *isd;
     F c;
@@ -1273,6 +1286,7 @@ struct ECheby1 : EpiBase<ECheby1<F, NV>, F>, NoFin {
 // (x_zero: x = 1*t, the ax_y branch of axpby).
 template <int NV>
 struct EProlongMixed : EpiBase<EProlongMixed<NV>, float>, NoFin {
+    static constexpr int KIND = TK_PLAIN;
     static constexpr size_t SCRATCH_A = sizeof(double);
     double *x;
     int x_zero;

@@ -223,10 +223,14 @@ constexpr uint64_t WIDE_MAX_VALUES = 1u << 20;  // rows * nv up to which it is a
 // copy's round trip is not hidden) and the run of consecutive tiles a block
 // takes (1, 4 or 16, or the plane walk where the matrix has a walk stride) are
 // timed with CUDA events on the caller's x, with the epilogue of the call at hand
-// writing into scratch vectors, once per matrix, precision and nv, outside any
-// graph capture; the fastest is kept in the matrix (DCsr::tuned). (Timed as y = A
-// x, a Chebyshev step or a prolongation got the shape that is best without its
-// epilogue's operands: 34 us against 26 for the 96^3 prolongation.) Matrices of at most WIDE_MAX_VALUES rows
+// writing into scratch vectors, once per matrix, kind of epilogue (TuneKind),
+// precision and nv, outside any graph capture; the fastest is kept in the matrix
+// (DCsr::tuned). (Timed as y = A x, a Chebyshev step or a prolongation got the shape
+// that is best without its epilogue's operands: 34 us against 26 for the 96^3
+// prolongation. Shared between all epilogues, the shape depended on which of them
+// ran first. One for every epilogue would measure three on each level: first solves
+// of 64^3 systems took 1.5 to 2.3 times as long, later ones were as fast.)
+// Matrices of at most WIDE_MAX_VALUES rows
 // times nv also time the warp-per-row kernel (code TUNE_WIDE). Every candidate
 // sums each (row, right-hand side) in the same CSR order, so the choice never
 // changes a result.
@@ -384,7 +388,7 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
         if (A.tune_on && aligned && (uintptr_t)x % 32 == 0) {
             int l = 0;
             while ((1 << l) < NV) ++l;
-            uint8_t &t = A.tuned[sizeof(F) == 4][sizeof(FX) == 4][l];
+            uint8_t &t = A.tuned[Epi::KIND][sizeof(F) == 4][sizeof(FX) == 4][l];
             if (!t) t = autotune<F, FX, I, NV, V>(A, x, epi, s);
             if (t == TUNE_WIDE) {
                 launch_wide<F, FX, I, NV, V>(A, x, epi, s);
@@ -487,7 +491,7 @@ static void launch_stencil(const DCsr &A, const F *x, const Epi &epi, cudaStream
 }
 
 // Stencil or CSR (DCsr::st_choice): on matrices with a grid-stencil copy and
-// tuning on, the first SpMV without dot products for each precision and nv
+// tuning on, the first SpMV without dot products for each kind, precision and nv
 // times the call at hand (its outputs into scratch vectors) with the stencil
 // kernel's two register budgets and with the CSR kernel's tuned shape (the
 // faster of two rounds of three launches each, outside any graph capture).
@@ -567,7 +571,7 @@ static void launch(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s) {
             if (A.tune_on) {
                 int l = 0;
                 while ((1 << l) < NV) ++l;
-                uint8_t &c = A.st_choice[sizeof(F) == 4][l];
+                uint8_t &c = A.st_choice[Epi::KIND][sizeof(F) == 4][l];
                 if (!c) c = tune_stencil<F, I, NV, CALLER_X>(A, x, epi, s);
                 if (c) choice = c;
             }

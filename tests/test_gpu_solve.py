@@ -358,6 +358,45 @@ def test_autotuned_spmv_same_results(gpu, stencil, edge, nv, f32):
     assert out[0][1]["iters"] == out[1][1]["iters"]
 
 
+@pytest.mark.parametrize("compress", [2, 3])
+def test_each_kind_of_spmv_is_tuned_for_itself(gpu, compress):
+    """The launch shapes measured for the smoother's steps and residuals on a level are
+    not taken for the plain products, nor the other way round: the first y = A x
+    after a solve measures its own (more than one launch), later products do not, and
+    all give the untuned bits."""
+    import torch
+    row, col, val = gpu.generate_diffusion(27, 14, 14, 14, 1.0, 1.0, 4)
+    n, nv = len(row) - 1, 8
+    b = np.random.default_rng(9).uniform(-1, 1, n * nv)
+    sm = {"method": "Chebyshev", "polynomial_order": 2}
+    S = {}
+    for tune in (0, 1):
+        params = {"solver": {"method": "MergedPBiCGStab", "max_iters": 100, "rel_tolerance": 1e-8,
+                             "abs_tolerance": 0, "gpu_spmv_tune": tune},
+                  "preconditioner": dict(MG_BASE, method="MultiGrid", gpu_precond_f32=1,
+                                         gpu_index_compress=compress, gpu_spmv_tune=tune),
+                  "pre_smoother": sm, "post_smoother": dict(sm),
+                  "coarse_grid_solver": {"method": "Direct"}}
+        S[tune] = gpu_solve(gpu, row, col, val, nv, params, b)[2]
+    x = torch.rand(n, nv, device="cuda")
+    for level in (0, 1):
+        rows = S[0].level_info(level, 3)["nrows"]
+        for mode in (0, 1):
+            y = {}
+            for tune in (0, 1):
+                counts = []
+                for _ in range(2):
+                    y[tune] = torch.ones(rows, nv, device="cuda")
+                    torch.cuda.synchronize()
+                    k0 = gpu.kernel_launches()
+                    S[tune].level_spmv(level, 3, x.data_ptr(), y[tune].data_ptr(), nv, mode)
+                    torch.cuda.synchronize()
+                    counts.append(gpu.kernel_launches() - k0)
+                assert counts[1] == 1, (level, mode, counts)
+                assert (counts[0] > 1) == (tune == 1 and mode == 0), (level, mode, counts)
+            assert torch.equal(y[0], y[1])
+
+
 @pytest.mark.parametrize("stencil,edge,nv,f32", [(27, 20, 8, True), (27, 18, 4, False),
                                                  (7, 22, 16, True), (27, 17, 2, False)])
 def test_plane_walk_spmv_same_results(gpu, oracle, stencil, edge, nv, f32):
