@@ -116,15 +116,18 @@ inline uint32_t walk_stride(const DCsr &A, uint64_t R) {
     return S >= 2 && ntiles >= 2 * S ? (uint32_t)S : 0u;
 }
 
-template <typename F, typename FX, typename I, int NV, int VK, int NRED, typename V = F,
-          class Epi>
-static void launch_vk(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s,
-                      uint32_t nbuf_force = 0, uint32_t run = 1) {
+// How a launch stages its tiles, and the blocks that run at once.
+struct SpmvPlan {
+    uint32_t cap, nbuf;
+    size_t smem;
+    uint64_t wave;
+};
+// nbuf_force 0: as above; 1, 2: that many buffers (2 only where they fit); 3: no
+// staging (every tile reads global memory)
+template <typename F, typename FX, typename I, int NV, int VK, int NRED, typename V, class Epi>
+static SpmvPlan plan_vk(const DCsr &A, cudaStream_t s, uint32_t nbuf_force) {
     constexpr uint32_t LIMIT1 = (96u * 1024u - 64u) / (uint32_t)(sizeof(V) + sizeof(I));
     constexpr int NT = k::CT / VK;
-    // the kernel forms x offsets c*NV + k and row indices in 32 bits
-    XG_REQUIRE(std::max(A.ncols, A.nrows) * (uint64_t)NV < (1ull << 32), XAMG_ERR_UNSUPPORTED,
-               "SpMV: x of 2^32 or more values");
     auto kern = k::k_spmv<F, FX, I, NV, VK, NRED, Epi, V>;
     static bool big_smem = false;  // one flag per instantiation
     if (!big_smem) {
@@ -132,7 +135,6 @@ static void launch_vk(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s
                                      (int)stage_buffer_bytes<V, I>(LIMIT1)));
         big_smem = true;
     }
-    // nbuf_force 3: no staging (every tile reads global memory)
     const uint32_t cap = nbuf_force == 3 ? 0u : std::min(tile_max(A, NV, s), LIMIT1);
     const size_t one = stage_buffer_bytes<V, I>(cap);
     const int res1 = resident_blocks(kern, NT, one);
@@ -145,20 +147,30 @@ static void launch_vk(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s
             res = res2;
         }
     }
-    const size_t smem = nbuf * one;
+    return SpmvPlan{cap, nbuf, nbuf * one, (uint64_t)res * (uint64_t)ctx().sms};
+}
+
+template <typename F, typename FX, typename I, int NV, int VK, int NRED, typename V = F,
+          class Epi>
+static void launch_vk(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s,
+                      uint32_t nbuf_force = 0, uint32_t run = 1) {
+    // the kernel forms x offsets c*NV + k and row indices in 32 bits
+    XG_REQUIRE(std::max(A.ncols, A.nrows) * (uint64_t)NV < (1ull << 32), XAMG_ERR_UNSUPPORTED,
+               "SpMV: x of 2^32 or more values");
+    const SpmvPlan p = plan_vk<F, FX, I, NV, VK, NRED, V, Epi>(A, s, nbuf_force);
     const uint64_t R = k::CT / NV;
     const uint64_t ntiles = (A.nrows + R - 1) / R;
-    const uint64_t wave = (uint64_t)res * (uint64_t)ctx().sms;
     uint32_t stride = 0;
     if (NRED == 0 && run == RUN_WALK) {
         stride = walk_stride(A, R);
-        run = (uint32_t)std::max<uint64_t>(1, (ntiles + wave - 1) / wave);
+        run = (uint32_t)std::max<uint64_t>(1, (ntiles + p.wave - 1) / p.wave);
     }
     if (NRED > 0 || run < 1) run = 1;
     const uint32_t B = NRED > 0 ? (uint32_t)k::canon_blocks(A.nrows, NV)
-                                : (uint32_t)std::min<uint64_t>((ntiles + run - 1) / run, wave);
-    const uint32_t P = (uint32_t)std::min<uint64_t>(B, wave);
-    kern<<<P, NT, smem, s>>>(A.args<F>(), x, epi, ctx().red(), cap, nbuf, B, run, stride);
+                                : (uint32_t)std::min<uint64_t>((ntiles + run - 1) / run, p.wave);
+    const uint32_t P = (uint32_t)std::min<uint64_t>(B, p.wave);
+    k::k_spmv<F, FX, I, NV, VK, NRED, Epi, V><<<P, k::CT / VK, p.smem, s>>>(
+        A.args<F>(), x, epi, ctx().red(), p.cap, p.nbuf, B, run, stride);
     XG_CUDA(cudaGetLastError());
     ++g_kernel_launches;
 }
@@ -290,27 +302,37 @@ static uint8_t autotune(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t
     float best = 1e30f;
     uint8_t code = 1;
     constexpr bool V8 = spmv_has_vk8<FX, NV, 0>() && VD != 8 && VA != 8;
-    // run index 3: the plane walk, where the matrix has one at this nv. Fewer
-    // tiles than SMs times four leave each block at most one tile whatever the
-    // shape: runs of tiles would only take blocks away, and a second buffer is
-    // never filled, so those candidates are left out (their timings differed
-    // by noise alone).
+    // Run index 3: the plane walk, where the matrix has one at this nv. Where a
+    // candidate's blocks all run at once with at most one tile each, runs of tiles
+    // would only take blocks away and a second buffer is never filled: such
+    // candidates are left out (their timings differ by noise alone), and two
+    // buffers where they do not fit.
     const uint64_t tiles = (A.nrows + k::CT / NV - 1) / (uint64_t)(k::CT / NV);
-    const bool few = tiles <= 4ull * (uint64_t)ctx().sms;
-    const int nruns = few ? 1 : walk_stride(A, (uint64_t)(k::CT / NV)) ? 4 : 3;
-    for (int alt = 0; alt < 3; ++alt)
-        for (uint32_t nb = 1; nb <= 3; ++nb)
-            for (int ri = 0; ri < nruns; ++ri) {
-                if ((alt == 1 && VA == VD) || (alt == 2 && !V8) || (few && nb == 2)) continue;
+    const int nruns = walk_stride(A, (uint64_t)(k::CT / NV)) ? 4 : 3;
+    for (int alt = 0; alt < 3; ++alt) {
+        if ((alt == 1 && VA == VD) || (alt == 2 && !V8)) continue;
+        auto with_vk = [&](auto &&f) {
+            if (alt == 2) {
+                if constexpr (V8) f(NVc<8>());
+            } else if (alt) {
+                f(NVc<VA>());
+            } else {
+                f(NVc<VD>());
+            }
+        };
+        for (uint32_t nb = 1; nb <= 3; ++nb) {
+            SpmvPlan p{};
+            with_vk([&](auto vk) {
+                p = plan_vk<F, FX, I, NV, decltype(vk)::value, 0, V, Epi>(A, s, nb);
+            });
+            const bool one_each = tiles <= p.wave;
+            if (nb == 2 && (one_each || p.nbuf < 2)) continue;
+            for (int ri = 0; ri < (one_each ? 1 : nruns); ++ri) {
                 const uint32_t run = ri == 3 ? RUN_WALK : TUNE_RUNS[ri];
                 auto go = [&] {
-                    if (alt == 2) {
-                        if constexpr (V8) launch_vk<F, FX, I, NV, 8, 0, V>(A, x, e, s, nb, run);
-                    } else if (alt) {
-                        launch_vk<F, FX, I, NV, VA, 0, V>(A, x, e, s, nb, run);
-                    } else {
-                        launch_vk<F, FX, I, NV, VD, 0, V>(A, x, e, s, nb, run);
-                    }
+                    with_vk([&](auto vk) {
+                        launch_vk<F, FX, I, NV, decltype(vk)::value, 0, V>(A, x, e, s, nb, run);
+                    });
                 };
                 // the faster of two rounds of three launches, after one untimed
                 float ms = 1e30f;
@@ -330,6 +352,8 @@ static uint8_t autotune(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t
                                    : (uint8_t)(1 + alt * 9 + (nb - 1) * 3 + ri);
                 }
             }
+        }
+    }
     if (A.nrows * (uint64_t)NV <= WIDE_MAX_VALUES) {
         auto go = [&] { launch_wide<F, FX, I, NV, V>(A, x, e, s); };
         float ms = 1e30f;
