@@ -331,7 +331,13 @@ __device__ __forceinline__ void stv(T *p, const Vec<T, VK> &o) {
         for (int v = 0; v < VK; ++v) p[v] = o.v[v];
     }
 }
-inline bool aligned16(const void *p) { return (uintptr_t)p % 16 == 0; }
+// Whether p allows ldv and stv of VK values: 16 bytes where those make up whole 16,
+// 8 where they are 8 (two floats), else the value's own size.
+template <int VK, typename T>
+inline bool aligned_for(const T *p) {
+    constexpr size_t B = VK * sizeof(T);
+    return (uintptr_t)p % (B % 16 == 0 ? 16 : B == 8 ? 8 : sizeof(T)) == 0;
+}
 
 // Register budget and gathers in flight, measured on the 27-point 128^3 matrix,
 // nv = 8 (us; gathers of up to 16 bytes, 1024 threads an SM and four entries at
@@ -900,7 +906,8 @@ struct EStore : EpiBase<EStore<F, NV>, F>, NoFin {
     static constexpr int KIND = TK_PLAIN;
     F *y;
     __host__ __device__ explicit EStore(F *y_) : y(y_) {}
-    bool aligned() const { return aligned16(y); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(y); }
     void redirect(void *a, void *) { y = (F *)a; }
     template <int VK>
     struct Pre {};
@@ -923,7 +930,8 @@ struct EAxpy : NoFin {
     static constexpr size_t SCRATCH_A = sizeof(F), SCRATCH_B = 0;
     F *y;
     __host__ __device__ explicit EAxpy(F *y_) : y(y_) {}
-    bool aligned() const { return aligned16(y); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(y); }
     void redirect(void *a, void *) { y = (F *)a; }
     template <int VK>
     struct Pre {
@@ -958,7 +966,8 @@ struct EResid : EpiBase<EResid<F, NV, NORM>, F> {
     const F *b;
     double *out;  // NORM: sums land here (nv values)
     EResid(F *r_, const F *b_, double *out_) : r(r_), b(b_), out(out_) {}
-    bool aligned() const { return aligned16(r) && aligned16(b); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(r) && aligned_for<VK>(b); }
     void redirect(void *a, void *) { r = (F *)a; }
     template <int VK>
     struct Pre {
@@ -994,6 +1003,7 @@ struct EGroup1 : EpiBase<EGroup1<NV>, double> {
     double *sc;
     EGroup1(double *r0_, double *p_, double *r_, const double *b_, double *sc_)
         : r0(r0_), p(p_), r(r_), b(b_), sc(sc_) {}
+    template <int VK>
     bool aligned() const { return true; }
     template <int VK>
     struct Pre {
@@ -1034,7 +1044,8 @@ struct EDotAlpha : EpiBase<EDotAlpha<NV>, double> {
     double *sc;
     __host__ __device__ EDotAlpha(double *v_, const double *r0_, double *sc_)
         : v(v_), r0(r0_), sc(sc_) {}
-    bool aligned() const { return aligned16(v) && aligned16(r0); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(v) && aligned_for<VK>(r0); }
     template <int VK>
     struct Pre {
         Vec<double, VK> r0;
@@ -1067,7 +1078,8 @@ struct EDot3 : EpiBase<EDot3<NV>, double> {
     const double *s;
     double *sc;
     __host__ __device__ EDot3(double *t_, const double *s_, double *sc_) : t(t_), s(s_), sc(sc_) {}
-    bool aligned() const { return aligned16(t) && aligned16(s); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(t) && aligned_for<VK>(s); }
     template <int VK>
     struct Pre {
         Vec<double, VK> s;
@@ -1115,7 +1127,8 @@ struct EJacobi : EpiBase<EJacobi<F, NV>, F>, NoFin {
     F relax;
     __host__ __device__ EJacobi(F *xout_, const F *xin_, const F *b_, const F *d_, F relax_)
         : xout(xout_), xin(xin_), b(b_), d(d_), relax(relax_) {}
-    bool aligned() const { return aligned16(xout) && aligned16(xin) && aligned16(b); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(xout) && aligned_for<VK>(xin) && aligned_for<VK>(b); }
     void redirect(void *a, void *) { xout = (F *)a; }
     template <int VK>
     struct Pre {
@@ -1149,7 +1162,8 @@ struct ECheby0 : EpiBase<ECheby0<F, NV>, F>, NoFin {
     F c;
     ECheby0(F *rs_, F *t1s_, const F *b_, const F *isd_, F c_)
         : rs(rs_), t1s(t1s_), b(b_), isd(isd_), c(c_) {}
-    bool aligned() const { return aligned16(rs) && aligned16(t1s) && aligned16(b); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(rs) && aligned_for<VK>(t1s) && aligned_for<VK>(b); }
     void redirect(void *a, void *c2) {
         rs = (F *)a;
         t1s = (F *)c2;
@@ -1246,7 +1260,8 @@ struct ECheby1 : EpiBase<ECheby1<F, NV>, F>, NoFin {
     int last, x_zero;
     ECheby1(F *out_, const F *rs_, const F *isd_, F c_, int last_, int x_zero_)
         : out(out_), rs(rs_), isd(isd_), c(c_), last(last_), x_zero(x_zero_) {}
-    bool aligned() const { return aligned16(out) && aligned16(rs); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(out) && aligned_for<VK>(rs); }
     void redirect(void *a, void *) { out = (F *)a; }
     template <int VK>
     struct Pre {
@@ -1291,7 +1306,8 @@ struct EProlongMixed : EpiBase<EProlongMixed<NV>, float>, NoFin {
     double *x;
     int x_zero;
     EProlongMixed(double *x_, int x_zero_) : x(x_), x_zero(x_zero_) {}
-    bool aligned() const { return aligned16(x); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(x); }
     void redirect(void *a, void *) { x = (double *)a; }
     template <int VK>
     struct Pre {
@@ -1404,9 +1420,10 @@ struct EGroup4 {
         }
         stv<VK>(r + e, rv);
     }
+    template <int VK>
     bool aligned() const {
-        return aligned16(s) && aligned16(t) && aligned16(r0) && aligned16(r) &&
-               (!XUPD || (aligned16(x) && aligned16(pa) && aligned16(sa)));
+        return aligned_for<VK>(s) && aligned_for<VK>(t) && aligned_for<VK>(r0) && aligned_for<VK>(r) &&
+               (!XUPD || (aligned_for<VK>(x) && aligned_for<VK>(pa) && aligned_for<VK>(sa)));
     }
     __device__ void operator()(int k, const double *s1) const {
         double *S = sc;
@@ -1473,7 +1490,8 @@ struct EPcgAp : EpiBase<EPcgAp<NV>, double> {
     const double *p;
     double *sc;
     EPcgAp(double *Ap_, const double *p_, double *sc_) : Ap(Ap_), p(p_), sc(sc_) {}
-    bool aligned() const { return aligned16(Ap) && aligned16(p); }
+    template <int VK>
+    bool aligned() const { return aligned_for<VK>(Ap) && aligned_for<VK>(p); }
     template <int VK>
     struct Pre {
         Vec<double, VK> p;

@@ -123,11 +123,11 @@ void group4(uint64_t n, const double *s_, const double *t, const double *r0, dou
         const k::EGroup4<NV, true> ex{s_, t, r0, r, x, pa, sa, sc};
         const k::EGroup4<NV, false> e{s_, t, r0, r, x, pa, sa, sc};
         // a caller's vectors (the kernel-level entry point) may be unaligned
-        if (with_x && ex.aligned())
+        if (with_x && ex.template aligned<VK>())
             launch_rows<double, NV, 1, VK>(n, ex, s);
         else if (with_x)
             launch_rows<double, NV, 1>(n, ex, s);
-        else if (e.aligned())
+        else if (e.template aligned<VK>())
             launch_rows<double, NV, 1, VK>(n, e, s);
         else
             launch_rows<double, NV, 1>(n, e, s);

@@ -378,10 +378,10 @@ static uint8_t autotune(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t
     return code;
 }
 
-// Vector loads need x aligned to VK elements and the epilogue's vectors to 16
-// bytes; library vectors always are (cudaMalloc). The entry points that take a
-// caller's vectors (CALLER_X) fall back to one right-hand side per thread where
-// they are not (same results, same reduction order).
+// Vector loads need x aligned to VK elements and the epilogue's vectors to their
+// accesses (aligned_for); library vectors always are (cudaMalloc). The entry points
+// that take a caller's vectors (CALLER_X) fall back to fewer right-hand sides per
+// thread where they are not (same results, same reduction order).
 template <typename F, typename FX, typename I, int NV, int NRED, bool CALLER_X, typename V,
           class Epi>
 static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s) {
@@ -390,8 +390,11 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
     constexpr int VK = NRED > 0 ? std::min(NV, 4) : k::spmv_vk<FX, NV>();
     // The widest gathers, 32 bytes, where nothing was measured for the matrix.
     constexpr int VW = std::min(NV, 32 / (int)sizeof(FX));
-    // the epilogue's vectors are read and written 16 bytes at a time too
-    const bool aligned = epi.aligned();
+    // whether x and the epilogue's vectors allow vk right-hand sides a thread
+    auto fits = [&](auto vkc) {
+        constexpr int vk = decltype(vkc)::value;
+        return vk == 1 || ((uintptr_t)x % (vk * sizeof(FX)) == 0 && epi.template aligned<vk>());
+    };
     if constexpr (NRED == 0) {
         if (A.wide_force && A.nrows * (uint64_t)NV <= WIDE_MAX_VALUES) {
             launch_wide<F, FX, I, NV, V>(A, x, epi, s);
@@ -403,55 +406,51 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
                 return;
             }
         if (A.walk_force && walk_stride(A, (uint64_t)(k::CT / NV)) &&
-            (VK == 1 || (aligned && (uintptr_t)x % (VK * sizeof(FX)) == 0))) {
+            fits(NVc<VK>())) {
             launch_vk<F, FX, I, NV, VK, NRED, V>(A, x, epi, s, 0, RUN_WALK);
             return;
         }
     }
     if constexpr (NRED == 0 && NV > 1) {
-        if (A.tune_on && aligned && (uintptr_t)x % 32 == 0) {
+        constexpr int VA = spmv_vk_alt<FX, NV>(), VT = std::max(VK, VA);
+        constexpr bool V8 = spmv_has_vk8<FX, NV, NRED>() && VT != 8;
+        if (A.tune_on && fits(NVc<VT>())) {
             int l = 0;
             while ((1 << l) < NV) ++l;
+            const bool fits8 = !V8 || fits(NVc<8>());
             uint8_t &t = A.tuned[Epi::KIND][sizeof(F) == 4][sizeof(FX) == 4][l];
-            if (!t) t = autotune<F, FX, I, NV, V>(A, x, epi, s);
+            if (!t && fits8) t = autotune<F, FX, I, NV, V>(A, x, epi, s);
             if (t == TUNE_WIDE) {
                 launch_wide<F, FX, I, NV, V>(A, x, epi, s);
                 return;
             }
-            if (t) {
-                const Tuned c = tuned_shape(t);
-                if constexpr (spmv_has_vk8<FX, NV, NRED>() && VK != 8 &&
-                              spmv_vk_alt<FX, NV>() != 8) {
-                    if (c.alt == 2) {
-                        launch_vk<F, FX, I, NV, 8, NRED, V>(A, x, epi, s, c.nbuf, c.run);
-                        return;
-                    }
-                }
+            const Tuned c = tuned_shape(t ? t : 1);
+            if (t && c.alt == 2 && fits8) {
+                if constexpr (V8) launch_vk<F, FX, I, NV, 8, NRED, V>(A, x, epi, s, c.nbuf, c.run);
+                return;
+            }
+            if (t && c.alt != 2) {
                 if (c.alt)
-                    launch_vk<F, FX, I, NV, spmv_vk_alt<FX, NV>(), NRED, V>(A, x, epi, s,
-                                                                           c.nbuf, c.run);
+                    launch_vk<F, FX, I, NV, VA, NRED, V>(A, x, epi, s, c.nbuf, c.run);
                 else
                     launch_vk<F, FX, I, NV, VK, NRED, V>(A, x, epi, s, c.nbuf, c.run);
                 return;
             }
         }
     }
-    auto fits = [&](int vk) {
-        return vk == 1 || (aligned && (uintptr_t)x % (vk * sizeof(FX)) == 0);
-    };
     if constexpr (NRED == 0 && VW != VK) {
-        if (fits(VW)) {
+        if (fits(NVc<VW>())) {
             launch_vk<F, FX, I, NV, VW, NRED, V>(A, x, epi, s);
             return;
         }
     }
     if constexpr (NRED > 0 && CALLER_X && VK * sizeof(FX) > 16) {
-        if (!fits(VK) && fits(VK / 2)) {
+        if (!fits(NVc<VK>()) && fits(NVc<VK / 2>())) {
             launch_vk<F, FX, I, NV, VK / 2, NRED, V>(A, x, epi, s);
             return;
         }
     }
-    if (fits(VK)) {
+    if (fits(NVc<VK>())) {
         launch_vk<F, FX, I, NV, VK, NRED, V>(A, x, epi, s);
     } else if constexpr (CALLER_X) {
         launch_vk<F, FX, I, NV, 1, NRED, V>(A, x, epi, s);

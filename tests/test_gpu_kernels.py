@@ -86,6 +86,26 @@ def test_spmv_unaligned_vectors(gpu, oracle, nv, f32, dx, dy):
         assert got[dy:].tobytes() == want.tobytes() and np.all(got[:dy] == 9.0)
 
 
+@pytest.mark.parametrize("dx,dy", [(2, 0), (0, 2), (2, 2), (1, 2)])
+def test_spmv_float_pairs_on_8_bytes(gpu, oracle, dx, dy):
+    """Two right-hand sides in FP32 need 8-byte boundaries only, both in x and in y."""
+    import torch
+    rng = np.random.default_rng(dx + 10 * dy)
+    n, nv = 900, 2
+    row, col, val = random_csr(n, n, rng)
+    x, y0 = (rng.standard_normal(n * nv).astype(np.float32) for _ in range(2))
+    A, keep = dev_csr(gpu, row, col, val, n, 2, True)
+    xb, xp = shifted(x, dx)
+    for mode in (0, 1):
+        yb, yp = shifted(y0, dy)
+        gpu.call("XAMG_b200_spmv", C.byref(A), xp, yp, nv, mode, None)
+        torch.cuda.synchronize()
+        want = oracle.csr_ax_y(row, col, val.astype(np.float32), x, nv,
+                               axpy_y=(y0 if mode == 1 else None))
+        got = yb.cpu().numpy()
+        assert got[dy:].tobytes() == want.tobytes() and np.all(got[:dy] == 9.0)
+
+
 def test_spmv_edge_cases(gpu, oracle):
     import torch
     rng = np.random.default_rng(11)
