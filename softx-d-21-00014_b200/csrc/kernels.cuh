@@ -387,10 +387,14 @@ inline bool aligned_for(const T *p) {
 //   (FP64 x); one dot 285 -> 246. Two right-hand sides a thread keep four gathers:
 //   six took 75 us for one dot of the 27-point 80^3 matrix at nv = 2 against 70, and
 //   more on short rows, whose leftover entries are a group of their own.
-template <typename FX, int VK, int NRED>
+// * Short rows (SHORT): a row's few gathers end before more of them could be in
+//   flight, so what counts is the threads: 1,024 an SM at 64 registers, although
+//   some kernels then spill a few words. y = A x of a 7-point 80^3 matrix in FP64
+//   at nv = 16 and 32: 60 and 117 us with 640 threads an SM, 48 and 89 with 1,024.
+template <typename FX, int VK, int NRED, int SHORT>
 constexpr int spmv_min_blocks() {
     if (NRED > 0) return VK > 1 ? 8 : 4;
-    return VK * sizeof(FX) >= 32 ? 5 * VK / 2 : 4 * VK;
+    return VK * sizeof(FX) >= 32 && !SHORT ? 5 * VK / 2 : 4 * VK;
 }
 template <typename FX, int VK, int NRED>
 constexpr int spmv_unroll() {
@@ -574,8 +578,8 @@ __device__ __forceinline__ uint32_t stage_shift(const T *arr, uint32_t j0) {
 // `run` consecutive tiles (run q to block q % gridDim.x), so that a block's
 // successive tiles share columns in its SM's L1.
 template <typename F, typename FX, typename I, int NV, int VK, int NRED, class Epi,
-          typename V = F>
-__global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED>())
+          typename V = F, int SHORT = 0>
+__global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED, SHORT>())
     k_spmv(CsrArgs<F> A, const FX *__restrict__ x, Epi epi, RedArgs ra, uint32_t cap,
            uint32_t nbuf, uint32_t B, uint32_t run = 1, uint32_t stride = 0) {
     constexpr int G = NV / VK;

@@ -124,11 +124,12 @@ struct SpmvPlan {
 };
 // nbuf_force 0: as above; 1, 2: that many buffers (2 only where they fit); 3: no
 // staging (every tile reads global memory)
-template <typename F, typename FX, typename I, int NV, int VK, int NRED, typename V, class Epi>
+template <typename F, typename FX, typename I, int NV, int VK, int NRED, typename V, class Epi,
+          int SHORT = 0>
 static SpmvPlan plan_vk(const DCsr &A, cudaStream_t s, uint32_t nbuf_force) {
     constexpr uint32_t LIMIT1 = (96u * 1024u - 64u) / (uint32_t)(sizeof(V) + sizeof(I));
     constexpr int NT = k::CT / VK;
-    auto kern = k::k_spmv<F, FX, I, NV, VK, NRED, Epi, V>;
+    auto kern = k::k_spmv<F, FX, I, NV, VK, NRED, Epi, V, SHORT>;
     static bool big_smem = false;  // one flag per instantiation
     if (!big_smem) {
         XG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -151,13 +152,13 @@ static SpmvPlan plan_vk(const DCsr &A, cudaStream_t s, uint32_t nbuf_force) {
 }
 
 template <typename F, typename FX, typename I, int NV, int VK, int NRED, typename V = F,
-          class Epi>
+          int SHORT = 0, class Epi>
 static void launch_vk(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s,
                       uint32_t nbuf_force = 0, uint32_t run = 1) {
     // the kernel forms x offsets c*NV + k and row indices in 32 bits
     XG_REQUIRE(std::max(A.ncols, A.nrows) * (uint64_t)NV < (1ull << 32), XAMG_ERR_UNSUPPORTED,
                "SpMV: x of 2^32 or more values");
-    const SpmvPlan p = plan_vk<F, FX, I, NV, VK, NRED, V, Epi>(A, s, nbuf_force);
+    const SpmvPlan p = plan_vk<F, FX, I, NV, VK, NRED, V, Epi, SHORT>(A, s, nbuf_force);
     const uint64_t R = k::CT / NV;
     const uint64_t ntiles = (A.nrows + R - 1) / R;
     uint32_t stride = 0;
@@ -169,7 +170,7 @@ static void launch_vk(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s
     const uint32_t B = NRED > 0 ? (uint32_t)k::canon_blocks(A.nrows, NV)
                                 : (uint32_t)std::min<uint64_t>((ntiles + run - 1) / run, p.wave);
     const uint32_t P = (uint32_t)std::min<uint64_t>(B, p.wave);
-    k::k_spmv<F, FX, I, NV, VK, NRED, Epi, V><<<P, k::CT / VK, p.smem, s>>>(
+    k::k_spmv<F, FX, I, NV, VK, NRED, Epi, V, SHORT><<<P, k::CT / VK, p.smem, s>>>(
         A.args<F>(), x, epi, ctx().red(), p.cap, p.nbuf, B, run, stride);
     XG_CUDA(cudaGetLastError());
     ++g_kernel_launches;
@@ -223,6 +224,20 @@ template <typename FX, typename V, int NV>
 static bool xs_usable(const DCsr &A, const FX *x) {
     return A.xs_nv == NV && (uintptr_t)x % (k::spmv_vk<FX, NV>() * sizeof(FX)) == 0 &&
            k::xs_smem_bytes<FX, V, NV>(A.xs_umax, A.xs_emax) <= 96u * 1024u;
+}
+
+// Whether a matrix's tiles have about equally many entries. With 32-byte gathers a
+// warp takes twice the rows that it takes with 16-byte ones and waits for the
+// longest of them. Measured where the widest won and lost (us, 16-byte against
+// 32-byte gathers, 512,000 rows): 27-point, largest tile 1.02 times the mean, FP64 nv
+// = 8 64 against 61, FP32 nv = 16 64 against 58; random rows of 0 to 120 entries,
+// 1.4 to 2.2 times the mean, FP64 nv = 8 203 against 230, FP32 nv = 16 185 against
+// 224. Rows of fewer than 16 entries on average gain either way (1 to 5 entries,
+// FP64 nv = 4: 21 against 17).
+static bool even_rows(const DCsr &A, int nv, cudaStream_t s) {
+    const uint64_t R = (uint64_t)k::CT / (uint64_t)nv;
+    const uint64_t ntiles = (A.nrows + R - 1) / R;
+    return (double)tile_max(A, nv, s) * (double)ntiles <= 1.15 * (double)A.nnz;
 }
 
 constexpr uint8_t TUNE_WIDE = 28;         // autotuner code of the warp-per-row kernel
@@ -388,7 +403,8 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
     // Dot products: four right-hand sides a thread (kernels.cuh, register
     // budget); two where a caller's x allows 16-byte gathers only.
     constexpr int VK = NRED > 0 ? std::min(NV, 4) : k::spmv_vk<FX, NV>();
-    // The widest gathers, 32 bytes, where nothing was measured for the matrix.
+    // The widest gathers, 32 bytes, where nothing was measured for the matrix and its
+    // rows are short or about as long as one another.
     constexpr int VW = std::min(NV, 32 / (int)sizeof(FX));
     // whether x and the epilogue's vectors allow vk right-hand sides a thread
     auto fits = [&](auto vkc) {
@@ -439,7 +455,13 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
         }
     }
     if constexpr (NRED == 0 && VW != VK) {
-        if (fits(NVc<VW>())) {
+        const bool short_rows = A.nnz < 16 * A.nrows;
+        if (fits(NVc<VW>()) && (short_rows || even_rows(A, NV, s))) {
+            if constexpr (CALLER_X && std::is_same<FX, double>::value && VW == 4)
+                if (short_rows) {
+                    launch_vk<F, FX, I, NV, VW, NRED, V, 1>(A, x, epi, s);
+                    return;
+                }
             launch_vk<F, FX, I, NV, VW, NRED, V>(A, x, epi, s);
             return;
         }

@@ -106,6 +106,32 @@ def test_spmv_float_pairs_on_8_bytes(gpu, oracle, dx, dy):
         assert got[dy:].tobytes() == want.tobytes() and np.all(got[:dy] == 9.0)
 
 
+@pytest.mark.parametrize("f32", [False, True])
+@pytest.mark.parametrize("nv", [4, 8, 16, 32])
+@pytest.mark.parametrize("rows", ["even", "short", "uneven"])
+def test_spmv_row_lengths(gpu, oracle, nv, f32, rows):
+    """Rows about as long as one another, short ones and uneven ones take different
+    gather widths and register budgets: the same sums."""
+    import torch
+    rng = np.random.default_rng(nv)
+    n = 1100
+    deg = {"even": np.full(n, 27), "short": rng.integers(0, 8, n),
+           "uneven": rng.integers(0, 60, n) * (rng.random(n) < 0.5)}[rows]
+    row = np.concatenate([[0], np.cumsum(deg)]).astype(np.uint32)
+    col = rng.integers(0, n, row[-1]).astype(np.uint32)
+    dt = np.float32 if f32 else np.float64
+    val, x = rng.standard_normal(row[-1]), rng.standard_normal(n * nv).astype(dt)
+    A, keep = dev_csr(gpu, row, col, val, n, 4, f32)
+    for mode in (0, 1):
+        y0 = rng.standard_normal(n * nv).astype(dt)
+        yd, xd = torch_dev(y0), torch_dev(x)
+        gpu.call("XAMG_b200_spmv", C.byref(A), xd.data_ptr(), yd.data_ptr(), nv, mode, None)
+        torch.cuda.synchronize()
+        want = oracle.csr_ax_y(row, col, val.astype(dt), x, nv,
+                               axpy_y=(y0 if mode == 1 else None))
+        assert yd.cpu().numpy().tobytes() == want.tobytes()
+
+
 def test_spmv_edge_cases(gpu, oracle):
     import torch
     rng = np.random.default_rng(11)
