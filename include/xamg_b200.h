@@ -242,7 +242,9 @@ int XAMG_b200_matrix_hierarchy_load(size_t mid, const char *path);
  * row stride ldc. mode 0: C FP32 = acc (+ bias[N] if not NULL); 1: C BF16 =
  * acc (+ bias); 2: C BF16 = max(acc + bias, 0); 3: C BF16 = acc where
  * aux[M][ld_aux] (BF16) > 0, else 0. M and N multiples of 128, K a multiple
- * of 64, pointers 16-byte aligned. */
+ * of 64, pointers 16-byte aligned. The sum over K may be split, by a rule on M, N,
+ * K and the GPU: the same rows may round differently in a product of another size.
+ * Calls of one size on one GPU round alike. */
 int XAMG_b200_gemm_bf16(uint64_t M, uint64_t N, uint64_t K, const void *A, const void *B,
                         void *C, uint64_t ldc, int mode, const float *bias, const void *aux,
                         uint64_t ld_aux, void *stream);
@@ -264,7 +266,9 @@ int XAMG_b200_gemm_shape(uint64_t M, uint64_t N, uint64_t K, int may_split, int 
  * the mean squared error. Widths and batches are multiples of 128. X, T, Y
  * are FP32 device arrays [batch][n_in] / [batch][n_out]. Parameters (and
  * gradients) are laid out W1^T [h][n_in], b1 [h], W2^T [h][h], b2 [h],
- * W3^T [n_out][h], b3 [n_out] in host FP32 arrays of *count values. */
+ * W3^T [n_out][h], b3 [n_out] in host FP32 arrays of *count values. A predict's
+ * products may split their sums (XAMG_b200_gemm_bf16), so its rounding may depend on
+ * the batch and differ from a training pass's forward, whose sums are never split. */
 int XAMG_b200_mlp_create(uint32_t n_in, uint32_t n_hidden, uint32_t n_out, uint64_t seed,
                          size_t *id);
 int XAMG_b200_mlp_destroy(size_t id);

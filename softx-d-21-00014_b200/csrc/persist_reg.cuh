@@ -3,10 +3,11 @@
 // registers and the block's matrix entries in shared memory.
 //
 // An iteration of a small system is latency: five exchanges between all blocks
-// (two products, three groups of dot products) and what lies between them.
-// k_pbicgstab_persist keeps the vectors in global memory and puts a grid
-// barrier (1.6 us) before every exchange's reads: 24.1 us an iteration on the
-// 32^3 Poisson system (128 blocks, nv = 1). Here every exchanged value carries
+// (two products, three groups of dot products), one more for every Jacobi sweep
+// after the first in each of the two preconditioner applications, and what lies
+// between them. k_pbicgstab_persist keeps the vectors in global memory and puts a
+// grid barrier (1.6 us) before every exchange's reads: 24.1 us an iteration on the
+// 32^3 Poisson system with two sweeps, seven exchanges (128 blocks, nv = 1). Here every exchanged value carries
 // the number of its exchange beside it, in one 16-byte access, and its readers
 // poll the value itself: a product waits for the x of its own entries and a
 // reduction for the blocks' partial sums, one store and one read through L2
