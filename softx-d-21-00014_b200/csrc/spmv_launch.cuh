@@ -317,12 +317,15 @@ static uint8_t autotune(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t
     float best = 1e30f;
     uint8_t code = 1;
     constexpr bool V8 = spmv_has_vk8<FX, NV, 0>() && VD != 8 && VA != 8;
-    // Run index 3: the plane walk, where the matrix has one at this nv. Where a
-    // candidate's blocks all run at once with at most one tile each, runs of tiles
-    // would only take blocks away and a second buffer is never filled: such
-    // candidates are left out (their timings differ by noise alone), and two
-    // buffers where they do not fit.
+    // Run index 3: the plane walk, where the matrix has one at this nv. Where the GPU
+    // has at most four tiles an SM and a candidate's blocks all run at once with one
+    // tile each, runs of tiles would only take blocks away and a second buffer is
+    // never filled: such candidates are left out, and two buffers where they do not
+    // fit. (With more tiles, runs of them win on some levels although the blocks
+    // would all run at once: left out there too, 96^3 and 64^3 solves took 1 to 2 %
+    // longer.)
     const uint64_t tiles = (A.nrows + k::CT / NV - 1) / (uint64_t)(k::CT / NV);
+    const bool few = tiles <= 4ull * (uint64_t)ctx().sms;
     const int nruns = walk_stride(A, (uint64_t)(k::CT / NV)) ? 4 : 3;
     for (int alt = 0; alt < 3; ++alt) {
         if ((alt == 1 && VA == VD) || (alt == 2 && !V8)) continue;
@@ -340,7 +343,7 @@ static uint8_t autotune(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t
             with_vk([&](auto vk) {
                 p = plan_vk<F, FX, I, NV, decltype(vk)::value, 0, V, Epi>(A, s, nb);
             });
-            const bool one_each = tiles <= p.wave;
+            const bool one_each = few && tiles <= p.wave;
             if (nb == 2 && (one_each || p.nbuf < 2)) continue;
             for (int ri = 0; ri < (one_each ? 1 : nruns); ++ri) {
                 const uint32_t run = ri == 3 ? RUN_WALK : TUNE_RUNS[ri];
