@@ -1967,9 +1967,10 @@ constexpr int LOOP_ABS = 0, LOOP_REL = 32, LOOP_CONV = 64, LOOP_ITERS = 96, LOOP
 // blocks at each barrier); every reduction is summed per canonical block in
 // tile order. Each step applies the same element operations, row sums and
 // canonical reductions as the separate kernels of Krylov::step_tail,
-// step_body and stepped, so the iterates are the same bit for bit.
+// step_body and stepped, so the iterates are the same bit for bit. Two right-hand
+// sides are held to 64 registers, four blocks an SM (persist.cu: fits_nv).
 template <int NV, typename I>
-__global__ void __launch_bounds__(CT, 1) k_pbicgstab_persist(CsrArgs<double> A, PersistArgs P) {
+__global__ void __launch_bounds__(CT, NV == 2 ? 4 : 1) k_pbicgstab_persist(CsrArgs<double> A, PersistArgs P) {
     constexpr int R = CT / NV;
     __shared__ double SCS[SC_COUNT * SC_STRIDE];
     __shared__ double st_abs[NV], st_rel[NV];

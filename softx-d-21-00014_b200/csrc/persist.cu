@@ -14,9 +14,16 @@ namespace ops {
 // nv x 4 values each.
 static int grid_of(int B, int share) { return (B + share - 1) / (share < 1 ? 1 : share); }
 
+// By its registers an SM holds four blocks at nv = 1, 2 and 32, three at 4 and 8, two
+// at 16. What the next block an SM would take is solved faster by the separate
+// launches at nv = 4 and 16 (one launch against separate ones, ms, two Jacobi sweeps:
+// 33^3 nv = 4 7-point 3.07 and 2.87, 27-point 3.51 and 2.62; 18^3 nv = 16 4.05 and
+// 2.31, 3.05 and 1.68), and at nv = 2 on long rows (42^3 27-point 3.73 and 3.05), but
+// not on short ones (39^3 and 42^3 7-point 2.36 and 3.11, 2.90 and 3.46).
 template <int NV, typename I>
-static bool fits_nv(uint64_t n, int share) {
-    const int B = k::canon_blocks(n, NV);
+static bool fits_nv(const DCsr &A, int share) {
+    const int B = k::canon_blocks(A.nrows, NV);
+    if (NV == 2 && A.nnz >= 16 * A.nrows && grid_of(B, share) > 3 * ctx().sms) return false;
     if ((uint64_t)B * NV * 8 > (uint64_t)k::BMAX * 32 * 4) return false;
     const int res = occupancy(k::k_pbicgstab_persist<NV, I>, k::CT, 0);
     return (uint64_t)res * (uint64_t)ctx().sms >= (uint64_t)grid_of(B, share);
@@ -24,7 +31,7 @@ static bool fits_nv(uint64_t n, int share) {
 
 bool pbicgstab_persist_fits(const DCsr &A, int nv, int share) {
     bool ok = false;
-    XG_DISPATCH(A, nv, { ok = fits_nv<NV, I>(A.nrows, share); });
+    XG_DISPATCH(A, nv, { ok = fits_nv<NV, I>(A, share); });
     return ok;
 }
 

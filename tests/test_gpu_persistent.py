@@ -103,3 +103,20 @@ def test_grid_barrier_wait_runs_out(gpu):
     b = np.ones(len(row) - 1)
     x, st, S = gpu_solve(gpu, row, col, val, 1, params("MergedPBiCGStab", True, 1), b)
     assert st["conv"].all()
+
+
+@pytest.mark.parametrize("stencil,nv,edge,one_launch", [(7, 2, 39, True), (27, 2, 39, False),
+                                                        (7, 2, 45, False), (27, 2, 36, True),
+                                                        (7, 4, 33, False), (7, 16, 18, False)])
+def test_systems_past_three_blocks_an_sm(gpu, stencil, nv, edge, one_launch):
+    """More canonical blocks than three an SM: one launch takes them on short rows at
+    nv = 2, the separate launches otherwise; the same bits either way."""
+    row, col, val = gpu.generate_diffusion(stencil, edge, edge, edge, 1.0, 1.0, 4)
+    n = len(row) - 1
+    b = np.random.default_rng(nv).uniform(-1, 1, n * nv)
+    x0, s0, _ = gpu_solve(gpu, row, col, val, nv, params("MergedPBiCGStab", True, 0), b)
+    k0 = gpu.kernel_launches()
+    x1, s1, _ = gpu_solve(gpu, row, col, val, nv, params("MergedPBiCGStab", True, 1), b)
+    assert (gpu.kernel_launches() - k0 < s1["iters"]) == one_launch
+    assert s0["iters"] == s1["iters"] and s1["conv"].all()
+    assert x0.tobytes() == x1.tobytes()
