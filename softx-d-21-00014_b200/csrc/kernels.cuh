@@ -152,85 +152,94 @@ __device__ __forceinline__ void canon_partial(T (&acc)[VK][NRED], const RedArgs 
     __syncthreads();  // wsum is free for the next canonical block
 }
 
-// canon_final: called by every thread once the partials of the block's canonical
-// blocks (first, first + step, ...) are written. Canonical blocks l, l+32, ... are
+// The sums of a launch from its blocks' partials: canonical blocks l, l+32, ... are
 // group l; its sum is formed in block order, and the groups are added by a full
-// butterfly: fin(k, sums of k).
+// butterfly: fin(k, sums of k). Two forms of the same sums:
 //
-// Few sums (at most one a warp, or six): the last block to finish forms them all, a
-// warp each, lane l group l. Many: the last block of each group sums its group, one
-// thread a sum, and the last of these adds the groups; one block forming them all
-// kept the launch waiting for NV*NRED*B loads from one SM (the three dot products
-// of 32 right-hand sides took 142 us with the SpMV's 70). The second round of
-// fences, tickets and loads is 5 to 10 us, which few sums do not win back: y = A x
-// with one dot product, 512,000 rows of one entry, nv = 1, 20.9 us in groups, 13.1
-// without (27,000 rows: 10.8 and 8.0). One fence and one round of tickets a launch
-// block, however many canonical blocks it has played.
+// Few sums (canon_few: at most one a warp, or six): canon_final, called by every
+// thread at the end of the launch block. The last block to finish forms them all, a
+// warp each, lane l group l.
+//
+// Many: canon_group, called by every thread after each of the block's canonical
+// blocks. The last canonical block of each group has its group summed, one thread a
+// sum, while other blocks still run, and the last group adds the groups; one block
+// forming them all kept the launch waiting for NV*NRED*B loads from one SM (the
+// three dot products of 32 right-hand sides took 142 us with the SpMV's 70). Drawn
+// at the end of the launch block instead, the tickets made y = A x with one dot
+// product 7 to 15 % slower at nv = 16 and 32 (27-point 80^3, nv = 32: 249 against
+// 271 us).
+//
+// The second round of fences, tickets and loads is 5 to 10 us, which few sums do not
+// win back: one dot product, 512,000 rows of one entry, nv = 1, 20.9 us in groups,
+// 13.1 without (27,000 rows: 10.8 and 8.0).
+template <int NO, int NT>
+__host__ __device__ constexpr bool canon_few() { return NO <= NT / 32 || NO <= 6; }
+
 template <typename T, int NV, int NRED, int NT, class Fin>
-__device__ __forceinline__ void canon_final(const RedArgs &ra, uint32_t first, uint32_t step,
-                                            uint32_t B, const Fin &fin) {
+__device__ __forceinline__ void canon_final(const RedArgs &ra, uint32_t B, const Fin &fin) {
     constexpr int NW = NT / 32, NO = NV * NRED;
     __shared__ T sums[NO];
     __shared__ int is_last;
     const T *part = (const T *)ra.part;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if constexpr (NO <= NW || NO <= 6) {
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) is_last = atomicAdd(&ra.ticket[0], 1u) == gridDim.x - 1;
-        __syncthreads();
-        if (!is_last) return;
-        __threadfence();
-        for (int o = warp; o < NO; o += NW) {
-            T a = T(0);
-            for (uint32_t bb = lane; bb < B; bb += RED_GROUPS)
-                a = add(a, ld_cg(&part[(size_t)bb * NO + o]));
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = atomicAdd(&ra.ticket[0], 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int o = warp; o < NO; o += NW) {
+        T a = T(0);
+        for (uint32_t bb = lane; bb < B; bb += RED_GROUPS)
+            a = add(a, ld_cg(&part[(size_t)bb * NO + o]));
 #pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) a = add(a, shfl_xor(a, off));
-            if (lane == 0) sums[o] = a;
-        }
-    } else {
-        __shared__ uint32_t full;  // groups that this block completes, a bit each
-        T *group = (T *)ra.groups;
-        const uint32_t ngroups = B < (uint32_t)RED_GROUPS ? B : (uint32_t)RED_GROUPS;
-        if (threadIdx.x == 0) full = 0u;
-        __threadfence();
-        __syncthreads();
-        for (uint32_t cb = first + threadIdx.x * step; cb < B; cb += NT * step) {
-            const uint32_t l = cb % RED_GROUPS, members = (B - l + RED_GROUPS - 1) / RED_GROUPS;
-            if (atomicAdd(&ra.ticket[RED_GROUP + l], 1u) == members - 1) atomicOr(&full, 1u << l);
-        }
-        __syncthreads();
-        const uint32_t mine = full;
-        if (!mine) return;
-        __threadfence();
-        for (uint32_t g = mine; g; g &= g - 1) {
-            const uint32_t l = (uint32_t)__ffs((int)g) - 1;
-            for (int o = threadIdx.x; o < NO; o += NT) {
-                T a = T(0);
+        for (int off = 16; off >= 1; off >>= 1) a = add(a, shfl_xor(a, off));
+        if (lane == 0) sums[o] = a;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) ra.ticket[0] = 0u;
+    for (int kk = threadIdx.x; kk < NV; kk += NT) fin(kk, &sums[kk * NRED]);
+}
+
+template <typename T, int NV, int NRED, int NT, class Fin>
+__device__ __forceinline__ void canon_group(const RedArgs &ra, uint32_t cb, uint32_t B,
+                                            const Fin &fin) {
+    constexpr int NW = NT / 32, NO = NV * NRED;
+    __shared__ T sums[NO];
+    __shared__ int is_last;
+    const T *part = (const T *)ra.part;
+    T *group = (T *)ra.groups;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t l = cb % RED_GROUPS, members = (B - l + RED_GROUPS - 1) / RED_GROUPS;
+    const uint32_t ngroups = B < (uint32_t)RED_GROUPS ? B : (uint32_t)RED_GROUPS;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) is_last = atomicAdd(&ra.ticket[RED_GROUP + l], 1u) == members - 1;
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
+    for (int o = threadIdx.x; o < NO; o += NT) {
+        T a = T(0);
 #pragma unroll 8
-                for (uint32_t bb = l; bb < B; bb += RED_GROUPS)
-                    a = add(a, ld_cg(&part[(size_t)bb * NO + o]));
-                group[l * NO + o] = a;
-            }
-            if (threadIdx.x == 0) ra.ticket[RED_GROUP + l] = 0u;
-        }
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            const uint32_t done = (uint32_t)__popc(mine);
-            is_last = atomicAdd(&ra.ticket[0], done) == ngroups - done;
-        }
-        __syncthreads();
-        if (!is_last) return;
-        __threadfence();
+        for (uint32_t bb = l; bb < B; bb += RED_GROUPS)
+            a = add(a, ld_cg(&part[(size_t)bb * NO + o]));
+        group[l * NO + o] = a;
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        ra.ticket[RED_GROUP + l] = 0u;
+        is_last = atomicAdd(&ra.ticket[0], 1u) == ngroups - 1;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    __threadfence();
 #pragma unroll 4
-        for (int o = warp; o < NO; o += NW) {
-            T a = (uint32_t)lane < ngroups ? ld_cg(&group[lane * NO + o]) : T(0);
+    for (int o = warp; o < NO; o += NW) {
+        T a = (uint32_t)lane < ngroups ? ld_cg(&group[lane * NO + o]) : T(0);
 #pragma unroll
-            for (int off = 16; off >= 1; off >>= 1) a = add(a, shfl_xor(a, off));
-            if (lane == 0) sums[o] = a;
-        }
+        for (int off = 16; off >= 1; off >>= 1) a = add(a, shfl_xor(a, off));
+        if (lane == 0) sums[o] = a;
     }
     __syncthreads();
     if (threadIdx.x == 0) ra.ticket[0] = 0u;
@@ -391,6 +400,8 @@ inline bool aligned_for(const T *p) {
 //   flight, so what counts is the threads: 1,024 an SM at 64 registers, although
 //   some kernels then spill a few words. y = A x of a 7-point 80^3 matrix in FP64
 //   at nv = 16 and 32: 60 and 117 us with 640 threads an SM, 48 and 89 with 1,024.
+//   Not where all tiles run at once anyway: 12^3 to 30^3, nv = 4, 4.3 and 5.2 us
+//   against 6.2.
 template <typename FX, int VK, int NRED, int SHORT>
 constexpr int spmv_min_blocks() {
     if (NRED > 0) return VK > 1 ? 8 : 4;
@@ -735,8 +746,11 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED, SHORT>(
         __syncthreads();  // every reader is done with this tile's buffer
         if (nbuf == 1 && threadIdx.x == 0 && more) issue(nxt.j0, tile_end(nxt.r0));
         if constexpr (NRED > 0)
-            if (!more || an.left != at.left)
+            if (!more || an.left != at.left) {
                 canon_partial<F, NV, NRED, VK>(acc, ra, at.left);
+                if constexpr (!canon_few<NV * NRED, CT / VK>())
+                    canon_group<F, NV, NRED, CT / VK>(ra, at.left, B, epi);
+            }
         at = an;
         an = ann;
         cur = nxt;
@@ -748,7 +762,8 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED, SHORT>(
         if (threadIdx.x == 0)
             for (uint32_t u = n_used; u < n_issued; ++u) mbar_wait(&mbar[u % nbuf], (u / nbuf) & 1u);
     }
-    if constexpr (NRED > 0) canon_final<F, NV, NRED, CT / VK>(ra, blockIdx.x, gridDim.x, B, epi);
+    if constexpr (NRED > 0 && canon_few<NV * NRED, CT / VK>())
+        canon_final<F, NV, NRED, CT / VK>(ra, B, epi);
 }
 
 // Warp-per-row SpMV for matrices with few rows (the coarse levels and their
@@ -889,7 +904,10 @@ __global__ void __launch_bounds__(CT / VK, 4 * VK) k_rows(uint64_t n, Epi epi, R
     }
     if constexpr (NRED > 0) {
         canon_partial<F, NV, NRED, VK>(acc, ra, blockIdx.x);
-        canon_final<F, NV, NRED, CT / VK>(ra, blockIdx.x, gridDim.x, gridDim.x, epi);
+        if constexpr (canon_few<NV * NRED, CT / VK>())
+            canon_final<F, NV, NRED, CT / VK>(ra, gridDim.x, epi);
+        else
+            canon_group<F, NV, NRED, CT / VK>(ra, blockIdx.x, gridDim.x, epi);
     }
 }
 
