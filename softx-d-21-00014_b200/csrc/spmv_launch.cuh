@@ -233,7 +233,8 @@ static bool xs_usable(const DCsr &A, const FX *x) {
 // = 8 64 against 61, FP32 nv = 16 64 against 58; random rows of 0 to 120 entries,
 // 1.4 to 2.2 times the mean, FP64 nv = 8 203 against 230, FP32 nv = 16 185 against
 // 224. Rows of fewer than 16 entries on average gain either way (1 to 5 entries,
-// FP64 nv = 4: 21 against 17).
+// FP64 nv = 4: 21 against 17), and so do 32 right-hand sides in FP32, where a warp
+// takes eight rows at most (uneven rows 316 against 302).
 static bool even_rows(const DCsr &A, int nv, cudaStream_t s) {
     const uint64_t R = (uint64_t)k::CT / (uint64_t)nv;
     const uint64_t ntiles = (A.nrows + R - 1) / R;
@@ -459,11 +460,15 @@ static void launch_v(const DCsr &A, const FX *x, const Epi &epi, cudaStream_t s)
     }
     if constexpr (NRED == 0 && VW != VK) {
         const bool short_rows = A.nnz < 16 * A.nrows;
-        if (fits(NVc<VW>()) && (short_rows || even_rows(A, NV, s))) {
+        if (fits(NVc<VW>()) && (short_rows || (NV == 32 && sizeof(FX) == 4) ||
+                                 even_rows(A, NV, s))) {
             if constexpr (CALLER_X && std::is_same<FX, double>::value && VW == 4)
                 if (short_rows) {
-                    launch_vk<F, FX, I, NV, VW, NRED, V, 1>(A, x, epi, s);
-                    return;
+                    const SpmvPlan p = plan_vk<F, FX, I, NV, VW, NRED, V, Epi>(A, s, 0);
+                    if ((A.nrows + k::CT / NV - 1) / (uint64_t)(k::CT / NV) > p.wave) {
+                        launch_vk<F, FX, I, NV, VW, NRED, V, 1>(A, x, epi, s);
+                        return;
+                    }
                 }
             launch_vk<F, FX, I, NV, VW, NRED, V>(A, x, epi, s);
             return;
