@@ -156,7 +156,7 @@ __device__ __forceinline__ void canon_partial(T (&acc)[VK][NRED], const RedArgs 
 // group l; its sum is formed in block order, and the groups are added by a full
 // butterfly: fin(k, sums of k). Two forms of the same sums:
 //
-// Few sums (canon_few: at most one a warp, or six): canon_final, called by every
+// Few sums (canon_few: at most six): canon_final, called by every
 // thread at the end of the launch block. The last block to finish forms them all, a
 // warp each, lane l group l.
 //
@@ -171,9 +171,10 @@ __device__ __forceinline__ void canon_partial(T (&acc)[VK][NRED], const RedArgs 
 //
 // The second round of fences, tickets and loads is 5 to 10 us, which few sums do not
 // win back: one dot product, 512,000 rows of one entry, nv = 1, 20.9 us in groups,
-// 13.1 without (27,000 rows: 10.8 and 8.0).
-template <int NO, int NT>
-__host__ __device__ constexpr bool canon_few() { return NO <= NT / 32 || NO <= 6; }
+// 13.1 without (27,000 rows: 10.8 and 8.0). With eight they do: a dot product at nv =
+// 8, 27,000 and 512,000 rows, 9.4 and 15.0 against 10.5 and 16.3.
+template <int NO>
+__host__ __device__ constexpr bool canon_few() { return NO <= 6; }
 
 template <typename T, int NV, int NRED, int NT, class Fin>
 __device__ __forceinline__ void canon_final(const RedArgs &ra, uint32_t B, const Fin &fin) {
@@ -748,7 +749,7 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED, SHORT>(
         if constexpr (NRED > 0)
             if (!more || an.left != at.left) {
                 canon_partial<F, NV, NRED, VK>(acc, ra, at.left);
-                if constexpr (!canon_few<NV * NRED, CT / VK>())
+                if constexpr (!canon_few<NV * NRED>())
                     canon_group<F, NV, NRED, CT / VK>(ra, at.left, B, epi);
             }
         at = an;
@@ -762,7 +763,7 @@ __global__ void __launch_bounds__(CT / VK, spmv_min_blocks<FX, VK, NRED, SHORT>(
         if (threadIdx.x == 0)
             for (uint32_t u = n_used; u < n_issued; ++u) mbar_wait(&mbar[u % nbuf], (u / nbuf) & 1u);
     }
-    if constexpr (NRED > 0 && canon_few<NV * NRED, CT / VK>())
+    if constexpr (NRED > 0 && canon_few<NV * NRED>())
         canon_final<F, NV, NRED, CT / VK>(ra, B, epi);
 }
 
@@ -904,7 +905,7 @@ __global__ void __launch_bounds__(CT / VK, 4 * VK) k_rows(uint64_t n, Epi epi, R
     }
     if constexpr (NRED > 0) {
         canon_partial<F, NV, NRED, VK>(acc, ra, blockIdx.x);
-        if constexpr (canon_few<NV * NRED, CT / VK>())
+        if constexpr (canon_few<NV * NRED>())
             canon_final<F, NV, NRED, CT / VK>(ra, gridDim.x, epi);
         else
             canon_group<F, NV, NRED, CT / VK>(ra, blockIdx.x, gridDim.x, epi);
